@@ -230,7 +230,8 @@ int launch_pass(VptContext* c, cudaStream_t s, int mode, uint32_t buf, uint32_t 
         tp.maj_in_smem = 1;
         smem = static_cast<size_t>(c->mx) * c->my * c->mz * sizeof(float);
     }
-    const int ctas = vpt::persistent_grid(c, threads, vpt::nrc_kernel_ptr(mode, grid_maj, surfaces), smem);
+    const int ctas = vpt::persistent_grid(
+        c, threads, vpt::nrc_kernel_ptr(mode, grid_maj, surfaces, tp.grid.st_values != nullptr), smem);
     vpt::launch_nrc_pass(tp, mode, grid_maj, surfaces, ctas, threads, smem, s);
     NRCP_CUDA(cudaGetLastError());
     if (stream_mode == 1 && spp > 0) {

@@ -70,6 +70,8 @@ struct VptContextImpl {
     float* d_dense = nullptr;
     int32_t* d_leaf_table = nullptr;
     float* d_leaf_values = nullptr;
+    int32_t* d_st_table = nullptr;   // stencil copy of the grid (Grid::st_table); absent = not built
+    float* d_st_values = nullptr;
     float* d_cell_maj = nullptr;
     float* d_maj = nullptr;          // majorant grid of the DDA (pooled cells)
     int32_t mx = 0, my = 0, mz = 0, maj_shift = 0;
@@ -130,7 +132,6 @@ int nrc_reseed_train_rng(VptContextImpl* c);
 int upload_sample_jumps(VptContextImpl* c, uint32_t count, cudaStream_t s);
 int generate_sky_texture(float4* out, int w, int h, const float* states, const float* solar, const float* cmf,
                          const float sun_dir[3], int include_disc);
-const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage);
 // Wavefront plain tracer: runs the passes of one launch on `s` (vpt_wavefront.cu).
 int wf_run(VptContextImpl* c, const TraceParams& tp, bool grid_majorant, size_t smem, cudaStream_t s);
 int wf_ensure(VptContextImpl* c, uint32_t slots);

@@ -228,6 +228,79 @@ __global__ void leaf_box_max_kernel(const float* __restrict__ values, const int3
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(mx));
 }
 
+// Slots of the 2x2x2 leaves that the 9^3 voxels from the first voxel of cell (cx, cy, cz) lie in:
+// lane b < 8 gets leaf (cx + (b >> 2), cy + ((b >> 1) & 1), cz + (b & 1)), -1 where there is none.
+__device__ __forceinline__ int32_t corner_leaf(const int32_t* __restrict__ table, int lx, int ly, int lz, int cx, int cy,
+                                               int cz, int b) {
+    const int x = cx + ((b >> 2) & 1), y = cy + ((b >> 1) & 1), z = cz + (b & 1);
+    if (b >= 8 || x < 0 || y < 0 || z < 0 || x >= lx || y >= ly || z >= lz) return -1;
+    return table[(static_cast<int64_t>(x) * ly + y) * lz + z];
+}
+
+// One warp per cell: a slot if any of the 9^3 voxels its stencils read is not zero. Slots are
+// handed out by an atomic, so their order varies; what a lookup reads does not. Bound by the
+// reads of the leaves (most cells of a sparse grid stop after their eight table entries).
+__global__ void stencil_table_kernel(const int32_t* __restrict__ table, const float* __restrict__ values, int lx, int ly,
+                                     int lz, int32_t* __restrict__ st_table, int32_t* __restrict__ cell_of_slot,
+                                     unsigned int* __restrict__ count) {
+    const int64_t cell = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const int sy = ly + 1, sz = lz + 1;
+    if (cell >= static_cast<int64_t>(lx + 1) * sy * sz) return;
+    const int cz = static_cast<int>(cell % sz) - 1;
+    const int cy = static_cast<int>((cell / sz) % sy) - 1;
+    const int cx = static_cast<int>(cell / (static_cast<int64_t>(sz) * sy)) - 1;
+    const int32_t leaf = corner_leaf(table, lx, ly, lz, cx, cy, cz, lane);
+    bool any = false;
+    if (__any_sync(0xffffffffu, leaf >= 0)) {
+        for (int q0 = 0; q0 < 729 && !any; q0 += 32) {
+            const int q = min(q0 + lane, 728);
+            const int dz = q % 9, dy = (q / 9) % 9, dx = q / 81;
+            const int32_t slot = __shfl_sync(0xffffffffu, leaf, ((dx >> 3) << 2) | ((dy >> 3) << 1) | (dz >> 3));
+            const bool nz = slot >= 0 && values[static_cast<int64_t>(slot) * 512 +
+                                                (((dx & 7) << 6) | ((dy & 7) << 3) | (dz & 7))] != 0.0f;
+            any = __any_sync(0xffffffffu, nz);
+        }
+    }
+    if (lane == 0) {
+        int32_t slot = -1;
+        if (any) {
+            slot = static_cast<int32_t>(atomicAdd(count, 1u));
+            cell_of_slot[slot] = static_cast<int32_t>(cell);
+        }
+        st_table[cell] = slot;
+    }
+}
+
+// One CTA of 256 threads per slot: the 9^3 voxels through shared memory, then 1024 16-byte
+// stores (half a stencil each, consecutive threads to consecutive addresses). Bound by the writes.
+__global__ void __launch_bounds__(256) stencil_fill_kernel(const int32_t* __restrict__ table,
+                                                           const float* __restrict__ values, int lx, int ly, int lz,
+                                                           const int32_t* __restrict__ cell_of_slot,
+                                                           float* __restrict__ st_values) {
+    __shared__ float s_v[729];
+    __shared__ int32_t s_leaf[8];
+    const int32_t cell = cell_of_slot[blockIdx.x];
+    const int sy = ly + 1, sz = lz + 1;
+    const int cz = cell % sz - 1, cy = (cell / sz) % sy - 1, cx = cell / (sz * sy) - 1;
+    if (threadIdx.x < 8) s_leaf[threadIdx.x] = corner_leaf(table, lx, ly, lz, cx, cy, cz, threadIdx.x);
+    __syncthreads();
+    for (int q = threadIdx.x; q < 729; q += 256) {
+        const int dz = q % 9, dy = (q / 9) % 9, dx = q / 81;
+        const int32_t slot = s_leaf[((dx >> 3) << 2) | ((dy >> 3) << 1) | (dz >> 3)];
+        s_v[q] = slot < 0 ? 0.0f
+                          : values[static_cast<int64_t>(slot) * 512 + (((dx & 7) << 6) | ((dy & 7) << 3) | (dz & 7))];
+    }
+    __syncthreads();
+    float4* out = reinterpret_cast<float4*>(st_values + static_cast<int64_t>(blockIdx.x) * 4096);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int t = h * 256 + threadIdx.x;  // voxel t >> 1, its x (t & 1) half
+        const float* p = s_v + ((t >> 7) + (t & 1)) * 81 + ((t >> 4) & 7) * 9 + ((t >> 1) & 7);
+        out[t] = make_float4(p[0], p[1], p[9], p[10]);
+    }
+}
+
 // renderer_scene.cpp:498-509: the reference scans index coordinates [min, max) of the
 // inclusive index box, i.e. every voxel but the last plane along each axis.
 __global__ void global_max_kernel(const float* __restrict__ dense, int nx, int ny, int nz, unsigned int* out) {
@@ -323,6 +396,20 @@ void leaf_box_max(const float* values, const int32_t* origins, int64_t slots, co
     const int blocks = static_cast<int>(std::min<int64_t>((total + 255) / 256, 152 * 16));
     leaf_box_max_kernel<<<blocks, 256, 0, s>>>(values, origins, total, make_int3(box_lo[0], box_lo[1], box_lo[2]),
                                                make_int3(box_hi[0], box_hi[1], box_hi[2]), out);
+}
+
+void stencil_table(const int32_t* leaf_table, const float* leaf_values, int lx, int ly, int lz, int32_t* st_table,
+                   int32_t* cell_of_slot, unsigned int* count, cudaStream_t s) {
+    const int64_t cells = static_cast<int64_t>(lx + 1) * (ly + 1) * (lz + 1);
+    cudaMemsetAsync(count, 0, sizeof(unsigned int), s);
+    stencil_table_kernel<<<static_cast<unsigned int>((cells + 7) / 8), 256, 0, s>>>(leaf_table, leaf_values, lx, ly, lz,
+                                                                                   st_table, cell_of_slot, count);
+}
+
+void stencil_fill(const int32_t* leaf_table, const float* leaf_values, int lx, int ly, int lz,
+                  const int32_t* cell_of_slot, unsigned int slots, float* st_values, cudaStream_t s) {
+    if (slots == 0) return;
+    stencil_fill_kernel<<<slots, 256, 0, s>>>(leaf_table, leaf_values, lx, ly, lz, cell_of_slot, st_values);
 }
 
 void global_max(const float* dense, int nx, int ny, int nz, unsigned int* out, cudaStream_t s) {

@@ -258,8 +258,9 @@ constexpr int kStreamsPerPixel = 0, kStreamsSampleParallel = 1, kStreamsRuntime 
 // BSDF, NEE also samples the emitting triangles and shadow rays test the triangles for
 // visibility (optix_pathtracing_kernels.cu:84-96, 176-195, 216-239, 268-275, 340-356;
 // renderer_kernel_common.h:72-124, 146-403), in the plain and the radiance-cache modes.
+// kStencil: the lookups read the grid's stencil copy (sample_stencil, TraceParams::grid.st_values).
 template <bool kGridMajorant, bool kLog, int kMode, int kStreams = kStreamsRuntime, bool kStage = false,
-          bool kSurfaces = false>
+          bool kSurfaces = false, bool kStencil = false>
 __global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsSampleParallel) || kMode != kModePlain) && !kSurfaces
                                       ? kPlainSampleParallelThreads
                                       : 128,
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsS
                                                                             : kPlainPerPixelCtasPerSm)
     plain_trace_kernel(const TraceParams P) {
     static_assert(!kSurfaces || !kStage, "surfaces: no leaf staging");
+    static_assert(!kStencil || !kStage, "leaf staging reads the leaves");
     const bool sample_parallel = kStreams == kStreamsRuntime ? P.stream_mode == 1 : kStreams == kStreamsSampleParallel;
     extern __shared__ __align__(128) float s_maj[];
     const Grid& g = P.grid;
@@ -1279,6 +1281,8 @@ __global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsS
         if constexpr (kStage) {
             density = P.density_coeff * sample_trilinear_staged(g, need_lookup, world_to_index(g, lookup_pos), leaf_cache,
                                                                  stage, P.leaf_stage_min, stage_timed_out);
+        } else if constexpr (kStencil) {
+            if (need_lookup) density = P.density_coeff * sample_stencil(g, world_to_index(g, lookup_pos), leaf_cache);
         } else {
             if (need_lookup) density = P.density_coeff * sample_trilinear(g, world_to_index(g, lookup_pos), leaf_cache);
         }
@@ -1452,91 +1456,75 @@ size_t plain_smem_bytes(size_t maj_bytes, bool leaf_stage, int threads) {
     return (maj_bytes + 127) / 128 * 128 + warps * (kLeafBytes + sizeof(uint64_t));
 }
 
+namespace {
+template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kSurfaces>
+const void* kernel_of(bool stencil) {
+    return stencil ? reinterpret_cast<const void*>(
+                         plain_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false, kSurfaces, true>)
+                   : reinterpret_cast<const void*>(
+                         plain_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false, kSurfaces, false>);
+}
+
+template <bool kLog, int kMode, int kStreams, bool kSurfaces>
+const void* kernel_of(bool grid_majorant, bool stencil) {
+    return grid_majorant ? kernel_of<true, kLog, kMode, kStreams, kSurfaces>(stencil)
+                         : kernel_of<false, kLog, kMode, kStreams, kSurfaces>(stencil);
+}
+
+void launch(const void* kernel, const TraceParams& p, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
+    void* args[] = {const_cast<TraceParams*>(&p)};
+    cudaLaunchKernel(kernel, dim3(grid_ctas), dim3(threads), args, smem, s);
+}
+}  // namespace
+
 // Logged launches (decision records for the parity tests) follow the stream layout at run time;
 // the production launches use a kernel compiled for their layout. Leaf staging exists for the
-// majorant-grid tracker on sample-parallel streams and for its logged form.
-const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage) {
+// majorant-grid tracker on sample-parallel streams and for its logged form. `stencil`: the grid has
+// its stencil copy (grids too large for one, and the caller's grid of an allocation-free launch,
+// do not).
+const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage, bool stencil) {
     if (leaf_stage && grid_majorant)
         return logged ? reinterpret_cast<const void*>(plain_trace_kernel<true, true, kModePlain, kStreamsRuntime, true>)
                       : reinterpret_cast<const void*>(
                             plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel, true>);
-    if (logged) return grid_majorant ? reinterpret_cast<const void*>(plain_trace_kernel<true, true, kModePlain>)
-                                     : reinterpret_cast<const void*>(plain_trace_kernel<false, true, kModePlain>);
-    if (sample_parallel)
-        return grid_majorant
-                   ? reinterpret_cast<const void*>(plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel>)
-                   : reinterpret_cast<const void*>(plain_trace_kernel<false, false, kModePlain, kStreamsSampleParallel>);
-    return grid_majorant ? reinterpret_cast<const void*>(plain_trace_kernel<true, false, kModePlain, kStreamsPerPixel>)
-                         : reinterpret_cast<const void*>(plain_trace_kernel<false, false, kModePlain, kStreamsPerPixel>);
+    if (logged) return kernel_of<true, kModePlain, kStreamsRuntime, false>(grid_majorant, stencil);
+    if (sample_parallel) return kernel_of<false, kModePlain, kStreamsSampleParallel, false>(grid_majorant, stencil);
+    return kernel_of<false, kModePlain, kStreamsPerPixel, false>(grid_majorant, stencil);
 }
 
 void launch_plain(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
-    dim3 grid(grid_ctas), block(threads);
-    const size_t sm = grid_majorant ? smem : 0;
-    if (p.leaf_stage_min > 0 && grid_majorant && (p.dlog || p.stream_mode == 1)) {
-        if (p.dlog)
-            plain_trace_kernel<true, true, kModePlain, kStreamsRuntime, true><<<grid, block, sm, s>>>(p);
-        else
-            plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel, true><<<grid, block, sm, s>>>(p);
-    } else if (p.dlog) {
-        if (grid_majorant)
-            plain_trace_kernel<true, true, kModePlain><<<grid, block, sm, s>>>(p);
-        else
-            plain_trace_kernel<false, true, kModePlain><<<grid, block, sm, s>>>(p);
-    } else if (p.stream_mode == 1) {
-        if (grid_majorant)
-            plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel><<<grid, block, sm, s>>>(p);
-        else
-            plain_trace_kernel<false, false, kModePlain, kStreamsSampleParallel><<<grid, block, sm, s>>>(p);
-    } else {
-        if (grid_majorant)
-            plain_trace_kernel<true, false, kModePlain, kStreamsPerPixel><<<grid, block, sm, s>>>(p);
-        else
-            plain_trace_kernel<false, false, kModePlain, kStreamsPerPixel><<<grid, block, sm, s>>>(p);
-    }
+    const bool stage = p.leaf_stage_min > 0 && grid_majorant && (p.dlog || p.stream_mode == 1);
+    const void* kernel = plain_kernel_ptr(grid_majorant, p.dlog != nullptr, p.stream_mode == 1, stage,
+                                          p.grid.st_values != nullptr);
+    launch(kernel, p, grid_ctas, threads, grid_majorant ? smem : 0, s);
 }
 
-template <bool kGridMajorant>
-static const void* surface_kernel_for(bool logged) {
-    return logged ? reinterpret_cast<const void*>(
-                        plain_trace_kernel<kGridMajorant, true, kModePlain, kStreamsRuntime, false, true>)
-                  : reinterpret_cast<const void*>(
-                        plain_trace_kernel<kGridMajorant, false, kModePlain, kStreamsRuntime, false, true>);
-}
-
-const void* surface_kernel_ptr(bool grid_majorant, bool logged) {
-    return grid_majorant ? surface_kernel_for<true>(logged) : surface_kernel_for<false>(logged);
+const void* surface_kernel_ptr(bool grid_majorant, bool logged, bool stencil) {
+    return logged ? kernel_of<true, kModePlain, kStreamsRuntime, true>(grid_majorant, stencil)
+                  : kernel_of<false, kModePlain, kStreamsRuntime, true>(grid_majorant, stencil);
 }
 
 void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
-    const size_t sm = grid_majorant ? smem : 0;
-    void* args[] = {const_cast<TraceParams*>(&p)};
-    cudaLaunchKernel(surface_kernel_ptr(grid_majorant, p.dlog != nullptr), dim3(grid_ctas), dim3(threads), args, sm, s);
+    launch(surface_kernel_ptr(grid_majorant, p.dlog != nullptr, p.grid.st_values != nullptr), p, grid_ctas, threads,
+           grid_majorant ? smem : 0, s);
 }
 
-template <int kMode, bool kSurfaces>
-static const void* nrc_kernel_for(bool grid_majorant) {
-    return grid_majorant
-               ? reinterpret_cast<const void*>(plain_trace_kernel<true, false, kMode, kStreamsRuntime, false, kSurfaces>)
-               : reinterpret_cast<const void*>(plain_trace_kernel<false, false, kMode, kStreamsRuntime, false, kSurfaces>);
+template <int kMode>
+static const void* nrc_kernel_for(bool grid_majorant, bool surfaces, bool stencil) {
+    return surfaces ? kernel_of<false, kMode, kStreamsRuntime, true>(grid_majorant, stencil)
+                    : kernel_of<false, kMode, kStreamsRuntime, false>(grid_majorant, stencil);
 }
 
-const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces) {
-    if (surfaces) {
-        if (mode == kModeTrainNrc) return nrc_kernel_for<kModeTrainNrc, true>(grid_majorant);
-        if (mode == kModeComboNrc) return nrc_kernel_for<kModeComboNrc, true>(grid_majorant);
-        return nrc_kernel_for<kModeRenderNrc, true>(grid_majorant);
-    }
-    if (mode == kModeTrainNrc) return nrc_kernel_for<kModeTrainNrc, false>(grid_majorant);
-    if (mode == kModeComboNrc) return nrc_kernel_for<kModeComboNrc, false>(grid_majorant);
-    return nrc_kernel_for<kModeRenderNrc, false>(grid_majorant);
+const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces, bool stencil) {
+    if (mode == kModeTrainNrc) return nrc_kernel_for<kModeTrainNrc>(grid_majorant, surfaces, stencil);
+    if (mode == kModeComboNrc) return nrc_kernel_for<kModeComboNrc>(grid_majorant, surfaces, stencil);
+    return nrc_kernel_for<kModeRenderNrc>(grid_majorant, surfaces, stencil);
 }
 
 void launch_nrc_pass(const TraceParams& p, int mode, bool grid_majorant, bool surfaces, int grid_ctas, int threads,
                      size_t smem, cudaStream_t s) {
-    const size_t sm = grid_majorant ? smem : 0;
-    void* args[] = {const_cast<TraceParams*>(&p)};
-    cudaLaunchKernel(nrc_kernel_ptr(mode, grid_majorant, surfaces), dim3(grid_ctas), dim3(threads), args, sm, s);
+    launch(nrc_kernel_ptr(mode, grid_majorant, surfaces, p.grid.st_values != nullptr), p, grid_ctas, threads,
+           grid_majorant ? smem : 0, s);
 }
 
 }  // namespace vpt

@@ -83,9 +83,9 @@ void launch_plain(const TraceParams& p, bool grid_majorant, int grid_ctas, int t
 // Dynamic shared memory of a plain launch: the staged majorant grid (`maj_bytes`, 0 if not
 // staged) and, with leaf staging, one 2 KB leaf buffer and one mbarrier per warp.
 size_t plain_smem_bytes(size_t maj_bytes, bool leaf_stage, int threads);
-const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage);
+const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage, bool stencil);
 // Plain tracer of scenes with surfaces (either stream layout, logged or not).
-const void* surface_kernel_ptr(bool grid_majorant, bool logged);
+const void* surface_kernel_ptr(bool grid_majorant, bool logged, bool stencil);
 void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s);
 // Threads per CTA of the plain tracer on sample-parallel streams and of the radiance-cache
 // passes without meshes (one CTA per SM); the other forms of the tracer run CTAs of 128 threads.
@@ -94,7 +94,7 @@ constexpr int kPlainSampleParallelThreads = 896;
 // pass; `surfaces`: the instance that also traces the context's triangle meshes.
 void launch_nrc_pass(const TraceParams& p, int mode, bool grid_majorant, bool surfaces, int grid_ctas, int threads,
                      size_t smem, cudaStream_t s);
-const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces);
+const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces, bool stencil);
 // Jump table of sample-parallel streams first .. first + count - 1, computed on the device.
 void launch_sample_jump_table(ulonglong2* out, uint32_t first, uint32_t count, cudaStream_t s);
 void launch_finalize_mean(const double* sum, float* mean, uint32_t n_values, uint32_t samples, cudaStream_t s);
