@@ -41,6 +41,7 @@ extern "C" {
 #define VPT_DEVERR_TRAIN_FULL 0x4u    /* the training-vertex buffer overflowed */
 #define VPT_DEVERR_STAGE_TIMEOUT 0x8u /* a leaf-staging copy did not complete in time (staging stopped) */
 #define VPT_DEVERR_BVH_STACK 0x10u    /* a surface BVH traversal ran out of stack (nodes skipped) */
+#define VPT_DEVERR_QUEUE_TIMEOUT 0x20u /* a work queue entry of the tracker did not arrive in time (paths dropped) */
 
 typedef struct VptContext VptContext;
 
@@ -390,13 +391,12 @@ int vpt_set_tracker(VptContext* ctx, int32_t kind, int32_t slots_per_sm, int32_t
  * the same leaf in one tracking step; those lanes read their stencils from it. 0 = off (the
  * default). Decisions and values are those of the unstaged tracker. */
 int vpt_set_leaf_staging(VptContext* ctx, int32_t min_lanes);
-/* Launch shape of the persistent tracker (CTAs per SM, threads per CTA, a multiple of 32 up to
- * 128) and the number of parked lanes of a warp that triggers its joint event phase; 0 = defaults:
- * one CTA of 896 threads per SM for the plain tracer on sample-parallel streams and for the
- * radiance-cache passes without meshes, as many 128-thread CTAs as fit for the other forms; park
- * threshold 16 for the plain tracer, 24 for the radiance-cache passes. Contexts whose launches run
- * concurrently on one GPU (several scenes at once) do better with 128-thread CTAs, which can share
- * an SM. */
+/* Launch shape of the persistent trackers: CTAs per SM, threads per CTA (a multiple of 32 up to
+ * 128), and the number of parked lanes of a warp that triggers its joint event phase (scenes with
+ * meshes and leaf staging only: the tracker of volume scenes has work queues instead); 0 = defaults:
+ * three CTAs of 256 threads per SM for volume scenes, as many 128-thread CTAs as fit for the other
+ * forms. Contexts whose launches run concurrently on one GPU (several scenes at once) do better with
+ * 128-thread CTAs, which can share an SM. */
 int vpt_set_launch_shape(VptContext* ctx, int32_t ctas_per_sm, int32_t threads_per_cta,
                          int32_t park_threshold);
 

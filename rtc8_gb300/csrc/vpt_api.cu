@@ -626,21 +626,17 @@ static int launch_plain_impl(VptContext* c, void* stream, uint32_t spp, uint32_t
     // Leaf staging: majorant-grid tracker on sample-parallel streams (and its logged form).
     const bool stage = c->leaf_stage_min > 0 && grid_maj && (dlog != nullptr || tp.stream_mode == 1) && !c->surf;
     tp.leaf_stage_min = stage ? c->leaf_stage_min : 0;
-    // One 896-thread CTA per SM for the production plain tracer on sample-parallel streams; the
-    // other forms (and leaf staging, whose per-warp buffers would exceed the default dynamic
-    // shared-memory limit at 28 warps) run CTAs of 128.
-    const bool sp_plain = dlog == nullptr && tp.stream_mode == 1 && !c->surf && c->tracker != 1 && !stage;
-    const int threads = c->threads > 0 ? c->threads : (sp_plain ? vpt::kPlainSampleParallelThreads : 128);
+    const int threads = c->threads > 0 ? c->threads : 128;  // of the surface tracer and with leaf staging
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) capture = cudaStreamCaptureStatusActive;
     if (c->surf) {
-        // Scenes with triangles: the surface form of the persistent tracker.
+        // Scenes with triangles: the surface tracer.
         const void* kernel = vpt::surface_kernel_ptr(grid_maj, dlog != nullptr, tp.grid.st_values != nullptr);
         int ctas = vpt::persistent_grid(c, threads, kernel, smem);
         vpt::launch_surface(tp, grid_maj, ctas, threads, smem, s);
     } else if (c->tracker == 1 && capture == cudaStreamCaptureStatusNone) {
         // Wavefront tracer: its passes are issued from the host until every slot retired (not
-        // capturable; a stream being captured gets the persistent megakernel below).
+        // capturable; a stream being captured gets one of the persistent trackers below).
         const uint64_t items = tp.stream_mode == 1 ? npix * spp : npix;
         const uint64_t per_sm = c->wf_slots_per_sm > 0 ? static_cast<uint64_t>(c->wf_slots_per_sm) : 3072u;
         const uint32_t slots = static_cast<uint32_t>(std::min<uint64_t>(items, per_sm * c->num_sms));
@@ -648,12 +644,13 @@ static int launch_plain_impl(VptContext* c, void* stream, uint32_t spp, uint32_t
         if (rc3) return rc3;
         rc3 = vpt::wf_run(c, tp, grid_maj, smem, s);
         if (rc3) return rc3;
+    } else if (stage) {
+        const size_t launch_smem = vpt::plain_smem_bytes(smem, true, threads);
+        const int ctas = vpt::persistent_grid(c, threads, vpt::stage_kernel_ptr(dlog != nullptr), launch_smem);
+        vpt::launch_stage(tp, ctas, threads, launch_smem, s);
     } else {
-        const size_t launch_smem = vpt::plain_smem_bytes(smem, stage, threads);
-        const void* kernel = vpt::plain_kernel_ptr(grid_maj, dlog != nullptr, tp.stream_mode == 1, stage,
-                                                   tp.grid.st_values != nullptr);
-        int ctas = vpt::persistent_grid(c, threads, kernel, launch_smem);
-        vpt::launch_plain(tp, grid_maj, ctas, threads, launch_smem, s);
+        VPT_CUDA(vpt::launch_queues(tp, vpt::kModePlain, grid_maj, c->threads > 0 ? c->threads : vpt::kQueueThreads,
+                                    c->ctas_per_sm, c->num_sms, s));
     }
     if (tp.stream_mode == 1)
         vpt::launch_finalize_mean_dev(c->d_sum, c->d_mean, static_cast<uint32_t>(3 * npix), c->d_frame, spp, s);

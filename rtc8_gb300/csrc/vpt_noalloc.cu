@@ -210,20 +210,11 @@ extern "C" int vpt_launch_plain_noalloc(const VptNoAllocTrace* a, void* stream) 
         return ctx_set_error(VPT_ERR_CUDA, "vpt_launch_plain_noalloc: clearing the scratch failed");
     if (tp.stream_mode == 1) launch_sample_jump_table(jumps, a->stream_base, a->spp, s);
 
-    const int threads = 128;
-    const bool grid_maj = f.majorant_mode == 1;
-    size_t smem = 0;
-    if (grid_maj && a->mx * a->my * a->mz <= kMajSmemCells) {
-        tp.maj_in_smem = 1;
-        smem = static_cast<size_t>(a->mx) * a->my * a->mz * sizeof(float);
-    }
-    int dev = 0, sms = 0, occ = 0;
+    int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return ctx_set_error(VPT_ERR_CUDA, "vpt_launch_plain_noalloc: device query failed");
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plain_kernel_ptr(grid_maj, false, tp.stream_mode == 1, false, false), threads, smem) != cudaSuccess ||
-        occ <= 0)
-        occ = 1;
-    launch_plain(tp, grid_maj, sms * occ, threads, smem, s);
+    if (launch_queues(tp, kModePlain, f.majorant_mode == 1, kQueueThreads, 0, sms, s) != cudaSuccess)
+        return ctx_set_error(VPT_ERR_CUDA, "vpt_launch_plain_noalloc: launch failed");
     if (tp.stream_mode == 1)
         launch_finalize_mean(a->sum_rgb, a->mean_rgb, static_cast<uint32_t>(3 * npix), a->accum_base + a->spp, s);
     if (cudaGetLastError() != cudaSuccess) return ctx_set_error(VPT_ERR_CUDA, "vpt_launch_plain_noalloc: launch failed");

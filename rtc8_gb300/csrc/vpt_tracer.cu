@@ -1,18 +1,18 @@
-// Persistent megakernel for the plain volumetric path tracer (the reference's pathTrace
-// ray-generation program, renderer/gpu_kernels/optix_pathtracing_kernels.cu:31-434 with
-// withNRC = generateTrainingData = false, for volume-only scenes).
+// Tracker with one path per lane: scenes with triangle meshes (plain and radiance-cache modes), and
+// the leaf-staging form of the volume tracer. Volume scenes run the tracker with work queues
+// (vpt_queues.cu), which gives the same paths. The reference is the pathTrace ray-generation
+// program and its radiance-cache forms (renderer/gpu_kernels/optix_pathtracing_kernels.cu:31-434).
 //
-// GB300 layout: one resident set of CTAs per SM pulls work items from a global counter (path
-// regeneration: a lane that finishes a path starts the next one at once). A work item is a
-// pixel (reference streams: its samples are traced in order so the pixel's PCG32 stream
-// advances exactly as in the reference) or one (pixel, sample) pair (sample-parallel streams).
-// Each loop iteration first lets every lane run its cheap, divergent event logic (camera ray,
-// vertex, Russian roulette, NEE set-up, phase sampling, accumulation, a bounded number of
-// majorant-grid cell steps) until it needs a density value, then all lanes perform their grid
-// lookups together, so the dominant gathers of delta and ratio tracking run converged. The
-// majorant grid is staged in shared memory when it fits.
+// One resident set of CTAs per SM pulls work items from a global counter (path regeneration: a
+// lane that finishes a path starts the next one at once). A work item is a pixel (reference
+// streams: its samples are traced in order so the pixel's PCG32 stream advances exactly as in the
+// reference) or one (pixel, sample) pair (sample-parallel streams). Each loop iteration first lets
+// every lane run its cheap, divergent event logic (camera ray, vertex, Russian roulette, NEE
+// set-up, phase sampling, accumulation, a bounded number of majorant-grid cell steps) until it
+// needs a density value, then all lanes perform their grid lookups together, so the gathers of
+// delta and ratio tracking run converged. The majorant grid is staged in shared memory when it fits.
 #include "vpt_ctx.h"
-#include "vpt_tracer.cuh"
+#include "vpt_track.cuh"
 
 namespace vpt {
 namespace {
@@ -31,53 +31,16 @@ enum : uint32_t {
     ST_NEE_SETUP,    // surface scenes: light sample and shadow ray of the current vertex
 };
 
-enum : uint32_t {
-    END_ESCAPE = 1,
-    END_RR = 2,
-    END_PDF_ZERO = 3,
-    END_MAX_BOUNCES = 4,
-    END_STEP_CAP = 5,
-    END_CACHE = 6,       // radiance-cache passes: ended with a cache query
-    END_TRAIN_FULL = 7,  // training pass: the training-vertex buffer was full
-};
-
-// Limits that apply even when the caller disables the configurable caps, so that no input
-// (zero or non-finite majorants, albedo 1 in a huge medium) can keep a launch running forever.
-constexpr uint32_t kHardStepCap = 1u << 24;
-constexpr uint32_t kHardVertexCap = 1u << 16;
-// Majorant-grid cells a lane crosses per tracking iteration before yielding to the warp. With
-// a pixel's samples traced consecutively (C2 / C5 ms per 16-spp launch, radiance-cache frame ms):
-// 8 -> 29.3 / 53.7 / 5.02, 16 -> 29.9 / 54.5 / -, 32 -> 29.5 / 54.6 / -; the radiance-cache passes
-// at 4 / 8 / 16: 5.08 / 5.02 / 5.01. Earlier, with the samples of all pixels interleaved (M paths/s):
-// 4 -> 454 / 927, 8 -> 471 / 979, 16 -> 480 / 977, 32 -> 481 / 974 (1 -> 4 had raised C2 by 12% with
-// IEEE division and libm-accurate functions).
-constexpr int kCellStepsPerPass = 8;
-constexpr int kNrcCellStepsPerPass = 8;
-constexpr int kSurfCellStepsPerPass = 16;
-// Parked lanes of a warp that trigger a joint event phase. Plain tracer, C2 / C5 / C1 ms per
-// 16-spp launch with a pixel's samples consecutive: 12 -> 30.6 / 55.4 / 1.13, 16 -> 29.6 / 54.6 /
-// 1.15, 20 -> 29.8 / 55.4 / 1.17, 24 -> 31.2 / 58.2 / 1.17, 28 -> 33.6 / 62.1 / 1.15 (with the samples
-// of all pixels interleaved 20 was best); the radiance-cache passes (shorter paths, more event
-// work per path) are fastest at 24 (frame 5.05 ms; 16 / 20 / 28 / 32: 5.31 / 5.09 / 5.06 / 5.23).
-constexpr int kParkThreshold = 16;
-// The surface tracer keeps the values it was tuned with (park threshold 20, 16 cells per step:
-// room scene 512^2 x 16 spp 92.8 ms per launch against 96.7 ms with the volume tracer's 16 and 8).
+// Majorant-grid cells a lane crosses per tracking iteration before yielding to the warp, and parked
+// lanes of a warp that trigger a joint event phase (room scene 512^2 x 16 spp: 92.8 ms per launch
+// at 16 cells and 20 lanes, 96.7 at 8 and 16).
+constexpr int kStageCellSteps = 8;
+constexpr int kSurfCellSteps = 16;
+constexpr int kStageParkThreshold = 16;
 constexpr int kSurfParkThreshold = 20;
 constexpr int kNrcParkThreshold = 24;
-// Resident CTAs per SM the register allocation is bounded for (CTAs of 128 threads unless noted).
-// The plain tracer on sample-parallel streams holds its state in 72 registers at 28 warps per SM
-// (1024^2 sparse 512^3 with 128-thread CTAs: 261 / 284 / 295 / 283 M paths/s at 5 / 6 / 7 / 8 per
-// SM). It runs them as ONE CTA of kPlainSampleParallelThreads = 896 threads per SM: one copy of
-// the staged majorant grid per SM instead of seven leaves more of the SM's L1 to the density
-// gathers (C2 / C5 / C1 per 16-spp launch: 35.0 / 68.4 / 1.17 ms as 7 x 128, 34.5 / 67.8 / 1.14
-// as 2 x 448, 34.0 / 67.0 / 1.13 as 1 x 896; 3 x 256 and 2 x 384, with more registers, slower).
-// Per-pixel streams (and the logged parity kernels) carry per-lane FP64 sums and stay at 5 CTAs
-// of 128, where they need no spills. The radiance-cache passes measured best at 7 x 128 (8 equal)
-// and better still as one 896-thread CTA per SM (256^2 frame: render pass 4.53 -> 4.44 ms, frame
-// 6.28 -> 6.13 ms); over meshes they keep CTAs of 128 (kSurfCtasPerSm).
-constexpr int kPlainCtasPerSm = 1;
-constexpr int kPlainPerPixelCtasPerSm = 5;
-constexpr int kNrcCtasPerSm = 1;
+// Resident CTAs of 128 threads per SM the register allocation is bounded for.
+constexpr int kStageCtasPerSm = 5;
 // The surface tracer carries the hit, the light sample's geometry and a BVH stack per lane; it
 // is latency-bound (every vertex traverses the BVH twice with divergent loops), and occupancy wins
 // over register spills: room scene 512^2 x 16 spp, 4 / 6 / 8 / 10 / 12 / 16 CTAs per SM ->
@@ -85,47 +48,6 @@ constexpr int kNrcCtasPerSm = 1;
 // 8 / 12 / 16 -> 110.7 / 102.4 / 96.7 ms; the same 2048 threads as 2 x 1024, 4 x 512 or 8 x 256
 // threads within 1%).
 constexpr int kSurfCtasPerSm = 16;
-
-struct DdaState {
-    int cell[3];
-    int step[3];
-    float tnext[3], tdelta[3];
-};
-
-// Majorant-grid DDA in index space. Cells are 2^maj_shift voxels wide; shared definition with
-// the oracle's restatement (overshooting a cell's exit restarts sampling at the exit).
-__device__ __forceinline__ void dda_init(const Grid& g, V3 eye, V3 dir, float t, DdaState* d) {
-    float o[3] = {(eye.x - g.origin[0]) * g.inv_voxel_size, (eye.y - g.origin[1]) * g.inv_voxel_size,
-                  (eye.z - g.origin[2]) * g.inv_voxel_size};
-    float dd[3] = {dir.x * g.inv_voxel_size, dir.y * g.inv_voxel_size, dir.z * g.inv_voxel_size};
-    int cdim[3] = {g.mx, g.my, g.mz};
-    const float size = static_cast<float>(1 << g.maj_shift);
-    const float inv_size = 1.0f / size;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float p = o[a] + dd[a] * t;
-        int c = static_cast<int>(floorf(p * inv_size));
-        c = min(max(c, 0), cdim[a] - 1);
-        d->cell[a] = c;
-        if (dd[a] > 0) {
-            d->step[a] = 1;
-            d->tnext[a] = ((c + 1) * size - o[a]) / dd[a];
-            d->tdelta[a] = size / dd[a];
-        } else if (dd[a] < 0) {
-            d->step[a] = -1;
-            d->tnext[a] = (c * size - o[a]) / dd[a];
-            d->tdelta[a] = -size / dd[a];
-        } else {
-            d->step[a] = 0;
-            d->tnext[a] = INFINITY;
-            d->tdelta[a] = INFINITY;
-        }
-    }
-}
-
-__device__ __forceinline__ float cell_maj(const float* maj, const Grid& g, const DdaState& d) {
-    return maj[(d.cell[0] * g.my + d.cell[1]) * g.mz + d.cell[2]];
-}
 
 enum : int { PASS_LOOKUP = 0, PASS_YIELD = 1, PASS_END = 2 };
 
@@ -135,10 +57,6 @@ enum : int { PASS_LOOKUP = 0, PASS_YIELD = 1, PASS_END = 2 };
 // exit (memoryless) and empty cells are crossed without draws, at most kCells crossings per
 // pass. PASS_LOOKUP leaves t at the tentative collision; PASS_END means the segment
 // is over (also on a NaN distance); PASS_YIELD means the pass crossed its cells without one.
-// The sign of a direction component: the DDA step along that axis (dda_init derives it from the
-// same sign, the index-space direction being the world direction times a positive scale).
-__device__ __forceinline__ int step_of(float d) { return d > 0 ? 1 : (d < 0 ? -1 : 0); }
-
 template <bool kGridMajorant, int kCells>
 __device__ __forceinline__ int track_pass(const Grid& g, const float* maj_grid, float density_coeff, float t1, V3 dir,
                                           Pcg32& rng, float& t, float& texit, float& maj, DdaState& dda,
@@ -181,75 +99,12 @@ __device__ __forceinline__ int track_pass(const Grid& g, const float* maj_grid, 
     }
 }
 
-// createRadianceQuery (optix_pathtracing_kernels.cu:14-29) for an in-medium vertex: position in
-// the world box (basic_types.h:2835-2838), normal = vOut as toPolarYUp outputs (the first slot
-// holds acos(y), the second the azimuth), roughness, diffuse = albedo, specular = 0.
-__device__ __forceinline__ void write_query(float* q, V3 pos, V3 vout, float roughness, float albedo, V3 wmin, V3 wmax) {
-    V3 d = wmax - wmin, r = pos - wmin;
-    float a, b;
-    to_polar_yup_sel(vout, &a, &b);
-    float2* p = reinterpret_cast<float2*>(q);
-    p[0] = make_float2(d.x != 0 ? r.x / d.x : 0.0f, d.y != 0 ? r.y / d.y : 0.0f);
-    p[1] = make_float2(d.z != 0 ? r.z / d.z : 0.0f, a);
-    p[2] = make_float2(b, a);
-    p[3] = make_float2(b, roughness);
-    p[4] = make_float2(albedo, albedo);
-    p[5] = make_float2(albedo, 0.0f);
-    p[6] = make_float2(0.0f, 0.0f);
-}
-
-// RadianceQuery of a surface vertex (optix_pathtracing_kernels.cu:14-29 with the BSDF's
-// getSurfaceParameters, common_renderer_types.h:1491-1496 Lambert, 1671-1677 dichromatic):
-// position in the world box, the shading normal and vOut as toPolarYUp outputs, roughness,
-// diffuse and specular reflectance of the material.
-__device__ __forceinline__ void write_query_surface(float* q, V3 pos, V3 normal, V3 vout, const SurfMaterial& m, V3 wmin,
-                                                    V3 wmax) {
-    V3 d = wmax - wmin, r = pos - wmin;
-    float na, nb, va, vb;
-    to_polar_yup_sel(normal, &na, &nb);
-    to_polar_yup_sel(vout, &va, &vb);
-    float2* p = reinterpret_cast<float2*>(q);
-    p[0] = make_float2(d.x != 0 ? r.x / d.x : 0.0f, d.y != 0 ? r.y / d.y : 0.0f);
-    p[1] = make_float2(d.z != 0 ? r.z / d.z : 0.0f, na);
-    p[2] = make_float2(nb, va);
-    p[3] = make_float2(vb, m.roughness);
-    p[4] = make_float2(m.diffuse[0], m.diffuse[1]);
-    p[5] = make_float2(m.diffuse[2], m.specular[0]);
-    p[6] = make_float2(m.specular[1], m.specular[2]);
-}
-
-// Work order of the training pass: item -> pixel of the training image, class by class, where
-// the class of a pixel is (its position in the 4x4 tile + offset) % 16 and class 0 holds the
-// unbiased suffixes (optix_pathtracing_kernels.cu:60-66). The long unbiased paths thus gather in
-// the first warps and CTAs, and the CTAs of the short biased suffixes retire early, freeing their
-// SM slots for the render pass that runs concurrently. Records stay at the reference's pixel
-// index; only the order in which the pixels are traced changes.
-__device__ __forceinline__ void train_item_to_pixel(uint32_t item, uint32_t w, uint32_t h, uint32_t offset,
-                                                    uint32_t* px, uint32_t* py) {
-    const uint32_t off = offset % 16;
-    for (uint32_t k = 0; k < 16; ++k) {
-        const uint32_t p = (k + 16 - off) % 16;  // tile position with (p + offset) % 16 == k
-        const uint32_t a = p % 4, b = p / 4;
-        const uint32_t cx = w > a ? (w - a + 3) / 4 : 0, cy = h > b ? (h - b + 3) / 4 : 0;
-        const uint32_t n = cx * cy;
-        if (item < n) {
-            *px = a + 4 * (item % cx);
-            *py = b + 4 * (item / cx);
-            return;
-        }
-        item -= n;
-    }
-    *px = 0;  // not reached for item < w * h
-    *py = 0;
-}
-
 // kMode: kModePlain (pathTrace), kModeRenderNrc (pathTraceWithNRC) or kModeTrainNrc
 // (generateTrainingData), optix_pathtracing_kernels.cu:438-448.
 // kStreams: the RNG stream layout the kernel is compiled for (kStreamsPerPixel,
 // kStreamsSampleParallel), or kStreamsRuntime to follow TraceParams::stream_mode. A fixed layout
 // drops the other layout's state (the per-lane FP64 sums and running mean of per-pixel streams)
 // from the register allocation.
-constexpr int kStreamsPerPixel = 0, kStreamsSampleParallel = 1, kStreamsRuntime = 2;
 
 // kStage: per-warp leaf staging in shared memory (sample_trilinear_staged; TraceParams::
 // leaf_stage_min lanes in one leaf trigger a bulk copy of that leaf).
@@ -261,13 +116,7 @@ constexpr int kStreamsPerPixel = 0, kStreamsSampleParallel = 1, kStreamsRuntime 
 // kStencil: the lookups read the grid's stencil copy (sample_stencil, TraceParams::grid.st_values).
 template <bool kGridMajorant, bool kLog, int kMode, int kStreams = kStreamsRuntime, bool kStage = false,
           bool kSurfaces = false, bool kStencil = false>
-__global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsSampleParallel) || kMode != kModePlain) && !kSurfaces
-                                      ? kPlainSampleParallelThreads
-                                      : 128,
-                                  kSurfaces                              ? kSurfCtasPerSm
-                                       : kMode != kModePlain                  ? kNrcCtasPerSm
-                                       : kStreams == kStreamsSampleParallel ? kPlainCtasPerSm
-                                                                            : kPlainPerPixelCtasPerSm)
+__global__ void __launch_bounds__(128, kSurfaces ? kSurfCtasPerSm : kStageCtasPerSm)
     plain_trace_kernel(const TraceParams P) {
     static_assert(!kSurfaces || !kStage, "surfaces: no leaf staging");
     static_assert(!kStencil || !kStage, "leaf staging reads the leaves");
@@ -300,7 +149,7 @@ __global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsS
     const uint32_t step_cap = P.max_steps > 0 ? static_cast<uint32_t>(P.max_steps) : kHardStepCap;
     const int park_threshold =
         P.park_threshold > 0 ? P.park_threshold
-                             : (kMode == kModePlain ? (kSurfaces ? kSurfParkThreshold : kParkThreshold) : kNrcParkThreshold);
+                             : (kMode == kModePlain ? (kSurfaces ? kSurfParkThreshold : kStageParkThreshold) : kNrcParkThreshold);
     const V3 bmin = v3(g.bbox_min[0], g.bbox_min[1], g.bbox_min[2]);
     const V3 bmax = v3(g.bbox_max[0], g.bbox_max[1], g.bbox_max[2]);
     // Sensor height of the launch's camera (optix_pathtracing_kernels.cu:43-55); the rest of the
@@ -766,8 +615,7 @@ __global__ void __launch_bounds__(((kMode == kModePlain && kStreams == kStreamsS
             }
             case ST_STEP: {
                 const V3 seg_dir = shadow ? -light_dir : dir;
-                constexpr int kCells = kMode == kModePlain ? (kSurfaces ? kSurfCellStepsPerPass : kCellStepsPerPass)
-                                                           : kNrcCellStepsPerPass;
+                constexpr int kCells = kMode == kModePlain && kSurfaces ? kSurfCellSteps : kStageCellSteps;
                 const int r = track_pass<kGridMajorant, kCells>(g, maj_grid, P.density_coeff, t1, seg_dir, rng, t, texit,
                                                                 maj, dda, n_cells);
                 if (r == PASS_LOOKUP) {
@@ -1457,18 +1305,13 @@ size_t plain_smem_bytes(size_t maj_bytes, bool leaf_stage, int threads) {
 }
 
 namespace {
-template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kSurfaces>
-const void* kernel_of(bool stencil) {
-    return stencil ? reinterpret_cast<const void*>(
-                         plain_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false, kSurfaces, true>)
-                   : reinterpret_cast<const void*>(
-                         plain_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false, kSurfaces, false>);
-}
-
-template <bool kLog, int kMode, int kStreams, bool kSurfaces>
-const void* kernel_of(bool grid_majorant, bool stencil) {
-    return grid_majorant ? kernel_of<true, kLog, kMode, kStreams, kSurfaces>(stencil)
-                         : kernel_of<false, kLog, kMode, kStreams, kSurfaces>(stencil);
+template <bool kLog, int kMode>
+const void* surface_kernel(bool grid_majorant, bool stencil) {
+    if (grid_majorant)
+        return stencil ? reinterpret_cast<const void*>(plain_trace_kernel<true, kLog, kMode, kStreamsRuntime, false, true, true>)
+                       : reinterpret_cast<const void*>(plain_trace_kernel<true, kLog, kMode, kStreamsRuntime, false, true, false>);
+    return stencil ? reinterpret_cast<const void*>(plain_trace_kernel<false, kLog, kMode, kStreamsRuntime, false, true, true>)
+                   : reinterpret_cast<const void*>(plain_trace_kernel<false, kLog, kMode, kStreamsRuntime, false, true, false>);
 }
 
 void launch(const void* kernel, const TraceParams& p, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
@@ -1477,31 +1320,18 @@ void launch(const void* kernel, const TraceParams& p, int grid_ctas, int threads
 }
 }  // namespace
 
-// Logged launches (decision records for the parity tests) follow the stream layout at run time;
-// the production launches use a kernel compiled for their layout. Leaf staging exists for the
-// majorant-grid tracker on sample-parallel streams and for its logged form. `stencil`: the grid has
-// its stencil copy (grids too large for one, and the caller's grid of an allocation-free launch,
-// do not).
-const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage, bool stencil) {
-    if (leaf_stage && grid_majorant)
-        return logged ? reinterpret_cast<const void*>(plain_trace_kernel<true, true, kModePlain, kStreamsRuntime, true>)
-                      : reinterpret_cast<const void*>(
-                            plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel, true>);
-    if (logged) return kernel_of<true, kModePlain, kStreamsRuntime, false>(grid_majorant, stencil);
-    if (sample_parallel) return kernel_of<false, kModePlain, kStreamsSampleParallel, false>(grid_majorant, stencil);
-    return kernel_of<false, kModePlain, kStreamsPerPixel, false>(grid_majorant, stencil);
+const void* stage_kernel_ptr(bool logged) {
+    return logged ? reinterpret_cast<const void*>(plain_trace_kernel<true, true, kModePlain, kStreamsRuntime, true>)
+                  : reinterpret_cast<const void*>(plain_trace_kernel<true, false, kModePlain, kStreamsSampleParallel, true>);
 }
 
-void launch_plain(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
-    const bool stage = p.leaf_stage_min > 0 && grid_majorant && (p.dlog || p.stream_mode == 1);
-    const void* kernel = plain_kernel_ptr(grid_majorant, p.dlog != nullptr, p.stream_mode == 1, stage,
-                                          p.grid.st_values != nullptr);
-    launch(kernel, p, grid_ctas, threads, grid_majorant ? smem : 0, s);
+void launch_stage(const TraceParams& p, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
+    launch(stage_kernel_ptr(p.dlog != nullptr), p, grid_ctas, threads, smem, s);
 }
 
 const void* surface_kernel_ptr(bool grid_majorant, bool logged, bool stencil) {
-    return logged ? kernel_of<true, kModePlain, kStreamsRuntime, true>(grid_majorant, stencil)
-                  : kernel_of<false, kModePlain, kStreamsRuntime, true>(grid_majorant, stencil);
+    return logged ? surface_kernel<true, kModePlain>(grid_majorant, stencil)
+                  : surface_kernel<false, kModePlain>(grid_majorant, stencil);
 }
 
 void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s) {
@@ -1509,21 +1339,15 @@ void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int
            grid_majorant ? smem : 0, s);
 }
 
-template <int kMode>
-static const void* nrc_kernel_for(bool grid_majorant, bool surfaces, bool stencil) {
-    return surfaces ? kernel_of<false, kMode, kStreamsRuntime, true>(grid_majorant, stencil)
-                    : kernel_of<false, kMode, kStreamsRuntime, false>(grid_majorant, stencil);
+const void* nrc_surface_kernel_ptr(int mode, bool grid_majorant, bool stencil) {
+    if (mode == kModeTrainNrc) return surface_kernel<false, kModeTrainNrc>(grid_majorant, stencil);
+    if (mode == kModeComboNrc) return surface_kernel<false, kModeComboNrc>(grid_majorant, stencil);
+    return surface_kernel<false, kModeRenderNrc>(grid_majorant, stencil);
 }
 
-const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces, bool stencil) {
-    if (mode == kModeTrainNrc) return nrc_kernel_for<kModeTrainNrc>(grid_majorant, surfaces, stencil);
-    if (mode == kModeComboNrc) return nrc_kernel_for<kModeComboNrc>(grid_majorant, surfaces, stencil);
-    return nrc_kernel_for<kModeRenderNrc>(grid_majorant, surfaces, stencil);
-}
-
-void launch_nrc_pass(const TraceParams& p, int mode, bool grid_majorant, bool surfaces, int grid_ctas, int threads,
-                     size_t smem, cudaStream_t s) {
-    launch(nrc_kernel_ptr(mode, grid_majorant, surfaces, p.grid.st_values != nullptr), p, grid_ctas, threads,
+void launch_nrc_surfaces(const TraceParams& p, int mode, bool grid_majorant, int grid_ctas, int threads, size_t smem,
+                         cudaStream_t s) {
+    launch(nrc_surface_kernel_ptr(mode, grid_majorant, p.grid.st_values != nullptr), p, grid_ctas, threads,
            grid_majorant ? smem : 0, s);
 }
 

@@ -1,4 +1,4 @@
-// Launch parameters and kernel declarations of the persistent volumetric tracker.
+// Launch parameters and kernel declarations of the persistent volumetric trackers.
 #pragma once
 
 #include "nrc_buffers.cuh"
@@ -79,22 +79,33 @@ struct TraceParams {
 // Majorant grids up to this many cells are staged in shared memory (32 KB).
 constexpr int kMajSmemCells = 8192;
 
-void launch_plain(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s);
-// Dynamic shared memory of a plain launch: the staged majorant grid (`maj_bytes`, 0 if not
-// staged) and, with leaf staging, one 2 KB leaf buffer and one mbarrier per warp.
+// Leaf-staging form of the plain tracer (majorant-grid mode; logged, or on sample-parallel streams).
+void launch_stage(const TraceParams& p, int grid_ctas, int threads, size_t smem, cudaStream_t s);
+// Dynamic shared memory of such a launch: the staged majorant grid (`maj_bytes`, 0 if not
+// staged), one 2 KB leaf buffer and one mbarrier per warp.
 size_t plain_smem_bytes(size_t maj_bytes, bool leaf_stage, int threads);
-const void* plain_kernel_ptr(bool grid_majorant, bool logged, bool sample_parallel, bool leaf_stage, bool stencil);
+const void* stage_kernel_ptr(bool logged);
 // Plain tracer of scenes with surfaces (either stream layout, logged or not).
 const void* surface_kernel_ptr(bool grid_majorant, bool logged, bool stencil);
 void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s);
-// Threads per CTA of the plain tracer on sample-parallel streams and of the radiance-cache
-// passes without meshes (one CTA per SM); the other forms of the tracer run CTAs of 128 threads.
-constexpr int kPlainSampleParallelThreads = 896;
+// The tracker with work queues (vpt_queues.cu): volume scenes, every mode, either stream layout.
+constexpr int kQueueThreads = 256;
+constexpr int kQueueCtasPerSm = 3;
+// Majorant grids up to this many cells are staged in each CTA's shared memory (512 cells: dense
+// 64^3 launch 0.747 -> 0.739 ms, radiance-cache frame 3.04 -> 2.99 ms; 4096 cells take the L1 from
+// the gathers, sparse 512^3 16.0 -> 19.0 ms).
+constexpr int kQueueMajCells = 1024;
+const void* queue_kernel_ptr(int mode, bool grid_majorant, bool logged, bool sample_parallel, bool stencil);
+// Dynamic shared memory of a launch of `threads` threads per CTA.
+size_t queue_smem_bytes(int mode, bool grid_majorant, bool logged, bool sample_parallel, int threads, size_t maj_bytes);
+// One launch with `threads` threads per CTA on `ctas_per_sm` x `sms` CTAs (0 = as many as fit).
+cudaError_t launch_queues(TraceParams& p, int mode, bool grid_majorant, int threads, int ctas_per_sm, int sms,
+                          cudaStream_t s);
 // Radiance-cache render (kModeRenderNrc), training (kModeTrainNrc) or combined (kModeComboNrc)
-// pass; `surfaces`: the instance that also traces the context's triangle meshes.
-void launch_nrc_pass(const TraceParams& p, int mode, bool grid_majorant, bool surfaces, int grid_ctas, int threads,
-                     size_t smem, cudaStream_t s);
-const void* nrc_kernel_ptr(int mode, bool grid_majorant, bool surfaces, bool stencil);
+// pass of a scene with triangle meshes.
+void launch_nrc_surfaces(const TraceParams& p, int mode, bool grid_majorant, int grid_ctas, int threads, size_t smem,
+                         cudaStream_t s);
+const void* nrc_surface_kernel_ptr(int mode, bool grid_majorant, bool stencil);
 // Jump table of sample-parallel streams first .. first + count - 1, computed on the device.
 void launch_sample_jump_table(ulonglong2* out, uint32_t first, uint32_t count, cudaStream_t s);
 void launch_finalize_mean(const double* sum, float* mean, uint32_t n_values, uint32_t samples, cudaStream_t s);
