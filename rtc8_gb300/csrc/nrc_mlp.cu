@@ -41,6 +41,8 @@ int fail(int code, const std::string& msg) {
         if (e_ != cudaSuccess) return fail(NRC_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+constexpr uint32_t kErrTimeout = 1u;
+
 constexpr int kTile = 128;
 constexpr int kWidth = 64;
 constexpr int kOutPad = 16;
@@ -306,6 +308,22 @@ __device__ __forceinline__ void encode_row_hashgrid(const NetLayout& ly, const u
     }
 }
 
+// The same input from features computed beforehand (grid_encode_kernel): f holds the 16 levels'
+// feature pairs, FP16.
+__device__ __forceinline__ void encode_row_features(const uint32_t (&f)[kGridLevels], const float* q, uint8_t* tile, int r) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        *reinterpret_cast<uint4*>(tile + cm_offset(r, k * 8, 64)) =
+            make_uint4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+#pragma unroll
+    for (int k = 4; k < 8; ++k) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = reference_feature(8 * k + i + 4, q);
+        store8(tile, r, k, 64, v);
+    }
+}
+
 // Adds the gradient of the 32 hash-grid features of one query (`d`, loss-scaled) into the FP32
 // table gradient: corner c of level lv receives w_c x d[2 lv + f].
 __device__ __forceinline__ void grid_backward(const NetLayout& ly, const float* q, const float (&d)[32],
@@ -438,9 +456,112 @@ __device__ __forceinline__ void load_row16(const uint8_t* tile, int r, int c0, i
     }
 }
 
-constexpr uint32_t kErrTimeout = 1u;
-
 __host__ __device__ __forceinline__ uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
+
+// ------------------------------------------------------------------------------ hash-grid features
+// Large inference batches compute the hash-grid features level by level: a CTA keeps ONE level's
+// table in shared memory (128 KB, brought in by one bulk copy) and takes a share of all positions
+// through it. Fused into the MLP kernel, the 128 corner gathers of a query go through the L1 in
+// requests of 32 different lines each (2^20 queries: 141 M L1 sectors, 268 us); from shared memory
+// a request of 32 random words takes about 3.4 cycles, and the 64 bytes of features per query travel
+// through the L2. The positions are gathered from the 56-byte records once, so that each level
+// reads 12 bytes per query. 2^20 queries: 264 -> 124 us (positions 12, features 70, MLP 40).
+constexpr int kEncodeThreads = 1024;
+constexpr uint32_t kFeatureChunk = 1u << 20;  // queries whose features (64 MB) are in flight: they stay in the L2
+
+__global__ void __launch_bounds__(256) grid_position_kernel(const float* __restrict__ in, uint32_t n,
+                                                            float* __restrict__ pos) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const float* q = in + static_cast<size_t>(i) * 14;
+    const float2 xy = __ldg(reinterpret_cast<const float2*>(q));
+    const float v[3] = {xy.x, xy.y, __ldg(q + 2)};
+    float p[3];
+    grid_position(v, p);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) pos[d * kFeatureChunk + i] = p[d];
+}
+
+// One level's feature pairs of positions first, first + step, .. < n, its table at shared address
+// `table`. Corners, weights and sums as in grid_corners and encode_row_hashgrid (same order of
+// operations, so the same bits); the index arithmetic is in bytes (hash and mask shifted by two), one
+// three-input operation per hashed corner (172 -> 107 instructions per query and level).
+template <bool kHashed>
+__device__ __forceinline__ void encode_level(const NetLayout& ly, uint32_t lv, uint32_t table, const float* __restrict__ pos,
+                                             uint32_t first, uint32_t step, uint32_t n, uint32_t* __restrict__ out) {
+    const float scale = ly.grid_scale[lv];
+    const uint32_t res = ly.grid_res[lv], size = ly.grid_size[lv], mask = (size - 1u) << 2;
+    float p[3] = {0.0f, 0.0f, 0.0f};
+    auto load = [&](uint32_t i) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) p[d] = i < n ? __ldg(pos + d * kFeatureChunk + i) : 0.0f;
+    };
+    load(first);
+    for (uint32_t i = first; i < n; i += step) {
+        float fr[3], om[3];
+        uint32_t g[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float v = fmaf(scale, p[d], 0.5f);
+            const float fl = floorf(v);
+            fr[d] = v - fl;
+            om[d] = 1.0f - fr[d];
+            g[d] = static_cast<uint32_t>(static_cast<int>(fl));
+        }
+        load(i + step);  // the next position while this one gathers
+        const float wxy[4] = {om[0] * om[1], fr[0] * om[1], om[0] * fr[1], fr[0] * fr[1]};
+        const uint32_t hy = g[1] * (2654435761u << 2), hz = g[2] * (805459861u << 2);
+        const uint32_t yz[4] = {hy ^ hz, (hy + (2654435761u << 2)) ^ hz, hy ^ (hz + (805459861u << 2)),
+                                (hy + (2654435761u << 2)) ^ (hz + (805459861u << 2))};
+        float f0 = 0.0f, f1 = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float w = wxy[c & 3] * ((c & 4) ? fr[2] : om[2]);
+            uint32_t e;
+            if constexpr (kHashed) {
+                e = (((g[0] + (c & 1)) << 2) ^ yz[c >> 1]) & mask;
+            } else {
+                e = g[0] + (c & 1) + (g[1] + ((c >> 1) & 1) + (g[2] + (c >> 2)) * res) * res;
+                e = (e >= size ? e - size : e) << 2;
+            }
+            uint32_t raw;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(raw) : "r"(table + e));
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&raw));
+            f0 += w * f.x;
+            f1 += w * f.y;
+        }
+        out[i] = pack_half2(f0, f1);
+    }
+}
+
+// features[level * kFeatureChunk + i] = the level's feature pair of position i (FP16), computed as
+// in encode_row_hashgrid. Bound by instruction issue and the shared-memory gathers.
+__global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const NetLayout ly, const uint32_t* __restrict__ grid,
+                                                                        const float* __restrict__ pos, uint32_t n,
+                                                                        uint32_t* __restrict__ features,
+                                                                        unsigned int* __restrict__ err) {
+    extern __shared__ __align__(128) uint32_t s_table[];
+    __shared__ uint64_t s_bar;
+    const uint32_t lv = blockIdx.x % kGridLevels, part = blockIdx.x / kGridLevels;
+    const uint32_t parts = gridDim.x / kGridLevels + (lv < gridDim.x % kGridLevels ? 1u : 0u);
+    if (threadIdx.x == 0) {
+        mbar_init(&s_bar, 1);
+        mbar_fence_init();
+        bulk_load(s_table, grid + ly.grid_off[lv], ly.grid_size[lv] * 4, &s_bar);
+    }
+    __syncthreads();
+    if (!__syncthreads_and(mbar_wait(&s_bar, 0))) {
+        if (threadIdx.x == 0) atomicOr(err, kErrTimeout);
+        mbar_wait(&s_bar, 0);  // again bounded: the copy must not land in another CTA's shared memory
+        return;
+    }
+    uint32_t* const out = features + static_cast<size_t>(lv) * kFeatureChunk;
+    const uint32_t first = part * kEncodeThreads + threadIdx.x, step = parts * kEncodeThreads;
+    if ((ly.grid_hashed >> lv) & 1u)
+        encode_level<true>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
+    else
+        encode_level<false>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
+}
 
 // ------------------------------------------------------------------------------ inference
 // G independent groups of 128 threads per CTA, each with its own 128-row tile, mbarrier and 64
@@ -455,7 +576,8 @@ __host__ __device__ constexpr uint32_t infer_tile_bytes(int in_dim) { return (kT
 // group's 64 accumulator columns) and feed the next layer's MMA as its A operand; only the encoded
 // input tile goes through shared memory.
 // idx (optional): row r of the launch is record idx[r] of `in` and `out`.
-template <int IN, int G, bool TA>
+// FEAT: the hash-grid features come from `grid` = the features of grid_encode_kernel.
+template <int IN, int G, bool TA, bool FEAT = false>
 __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout ly, const uint8_t* __restrict__ blob,
                                                              const uint32_t* __restrict__ grid,
                                                              const float* __restrict__ in,
@@ -493,15 +615,28 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
     uint32_t phase = 0;
     bool ok = true;
     float q[14];
+    uint32_t f[FEAT ? kGridLevels : 1];
+    auto load_features = [&](uint32_t row) {
+        if constexpr (FEAT) {
+#pragma unroll
+            for (int lv = 0; lv < kGridLevels; ++lv)
+                f[lv] = row < n ? __ldg(grid + static_cast<size_t>(lv) * kFeatureChunk + row) : 0u;
+        }
+    };
     const uint32_t stride = gridDim.x * G;
     load_query(in, idx, (blockIdx.x * G + g) * kTile + gt, n, q);
+    load_features((blockIdx.x * G + g) * kTile + gt);
     for (uint32_t tile = blockIdx.x * G + g; tile < ntiles && ok; tile += stride) {
         const uint32_t row = tile * kTile + gt;
-        encode_row<IN>(ly, grid, q, s_t, gt);
+        if constexpr (FEAT)
+            encode_row_features(f, q, s_t, gt);
+        else
+            encode_row<IN>(ly, grid, q, s_t, gt);
         // The next tile's queries load while this tile runs through the layers. (Encoding it
         // during layer 1, when the input tile is already free in the TA form, measured slower:
         // the group's next epilogue waits for the encoder.)
         load_query(in, idx, (tile + stride) * kTile + gt, n, q);
+        load_features((tile + stride) * kTile + gt);
         fence_async_smem();
         named_sync(bar_id, kTile);
         for (int j = 0; j < ly.L && ok; ++j) {
@@ -978,17 +1113,22 @@ int infer_groups(const NetLayout& l) {
         if (infer_smem(l, g) <= kMaxSmemOptIn) return g;
     return 1;
 }
-const void* infer_kernel_ptr(int enc, int groups) {
-    const bool vol = enc == NRC_ENCODING_VOLUME;
-    switch (groups) {
-    case 4: return vol ? reinterpret_cast<const void*>(mlp_infer_kernel<144, 4, kInferTmemActivations>)
-                       : reinterpret_cast<const void*>(mlp_infer_kernel<64, 4, kInferTmemActivations>);
-    case 2: return vol ? reinterpret_cast<const void*>(mlp_infer_kernel<144, 2, kInferTmemActivations>)
-                       : reinterpret_cast<const void*>(mlp_infer_kernel<64, 2, kInferTmemActivations>);
-    default: return vol ? reinterpret_cast<const void*>(mlp_infer_kernel<144, 1, kInferTmemActivations>)
-                        : reinterpret_cast<const void*>(mlp_infer_kernel<64, 1, kInferTmemActivations>);
-    }
+// Inference batches from this size on compute the hash-grid features level by level (us, fused
+// kernel against this: 16,384 queries 22.8 / 18.7, 65,536 24.7 / 20.8, 131,072 43.4 / 27.3, 2^20
+// 264 / 124, 3 M 730 / 358). Below it, three launches and 152 table loads are not worth it.
+constexpr uint32_t kFeatureMinQueries = 1u << 14;
+template <int G>
+const void* infer_kernel_for(int enc, bool features) {
+    if (enc == NRC_ENCODING_VOLUME) return reinterpret_cast<const void*>(mlp_infer_kernel<144, G, kInferTmemActivations>);
+    return features ? reinterpret_cast<const void*>(mlp_infer_kernel<64, G, kInferTmemActivations, true>)
+                    : reinterpret_cast<const void*>(mlp_infer_kernel<64, G, kInferTmemActivations>);
 }
+const void* infer_kernel_ptr(int enc, int groups, bool features) {
+    return groups == 4 ? infer_kernel_for<4>(enc, features)
+                       : (groups == 2 ? infer_kernel_for<2>(enc, features) : infer_kernel_for<1>(enc, features));
+}
+constexpr uint32_t kEncodeSmem = kGridMaxEntries * 4;
+constexpr size_t kFeatureBytes = static_cast<size_t>(kFeatureChunk) * (3 + kGridLevels) * 4;
 uint32_t train_smem(const NetLayout& l) {
     return align_up(l.blob_bytes, 1024) + kTile * l.in_dim * 2 + (l.L - 1) * kTile * kWidth * 2 +
            2 * kTile * kWidth * 2 + kTile * kOutPad * 2 + 2048 + 16;
@@ -1008,6 +1148,9 @@ struct NrcHandle {
     uint8_t *blob_train = nullptr, *blob_infer = nullptr;
     __half *grid_train = nullptr, *grid_infer = nullptr;  // FP16 hash-grid tables (hash grid only)
     unsigned int* err = nullptr;
+    // Workspaces of large hash-grid inference batches: taken and given back in stream order, so that
+    // calls on several streams each have their own.
+    cudaMemPool_t pool = nullptr;
     uint64_t steps = 0;
     int total_params() const { return ly.nparams + ly.grid_params; }
     const uint32_t* grid_words(bool train) const {
@@ -1129,12 +1272,33 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     }
     const bool vol = cfg->encoding == NRC_ENCODING_VOLUME;
     h->infer_groups = infer_groups(h->ly);
-    if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups), infer_smem(h->ly, h->infer_groups))) ||
+    if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, false), infer_smem(h->ly, h->infer_groups))) ||
         (rc = set_kernel_smem(vol ? reinterpret_cast<const void*>(mlp_train_kernel<144>)
                                   : reinterpret_cast<const void*>(mlp_train_kernel<64>),
                               train_smem(h->ly)))) {
         nrc_destroy(h);
         return rc;
+    }
+    if (cfg->encoding == NRC_ENCODING_HASHGRID) {
+        if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, true),
+                                  infer_smem(h->ly, h->infer_groups))) ||
+            (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel), kEncodeSmem))) {
+            nrc_destroy(h);
+            return rc;
+        }
+        // The pool keeps its memory between calls; the first workspace is reserved here. Without it
+        // (little memory left) large batches run the fused kernel.
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = UINT64_MAX;
+        void* work = nullptr;
+        if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+            cudaMallocFromPoolAsync(&work, kFeatureBytes, h->pool, 0) != cudaSuccess ||
+            cudaFreeAsync(work, 0) != cudaSuccess)
+            cudaGetLastError();
     }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         nrc_destroy(h);
@@ -1157,7 +1321,40 @@ int nrc_destroy(NrcHandle* h) {
     cudaFree(h->grid_train);
     cudaFree(h->grid_infer);
     cudaFree(h->err);
+    if (h->pool) cudaMemPoolDestroy(h->pool);
     delete h;
+    return NRC_OK;
+}
+
+static int launch_infer(NrcHandle* h, cudaStream_t s, const uint32_t* grid_or_features, bool features, const float* in,
+                        const uint32_t* idx, const uint32_t* dev_n, uint32_t n, float* out) {
+    const int G = h->infer_groups;
+    const uint32_t tiles = (n + kTile - 1) / kTile;
+    const uint32_t grid = std::min<uint32_t>((tiles + G - 1) / G, static_cast<uint32_t>(h->num_sms));
+    const uint8_t* blob = h->blob_infer;
+    unsigned int* err = h->err;
+    void* args[] = {&h->ly, &blob, &grid_or_features, &in, &idx, &dev_n, &n, &out, &err};
+    NRC_CUDA(cudaLaunchKernel(infer_kernel_ptr(h->cfg.encoding, G, features), dim3(grid), dim3(kTile * G), args,
+                              infer_smem(h->ly, G), s));
+    return NRC_OK;
+}
+
+// A batch of hash-grid queries, level by level and chunk by chunk (grid_encode_kernel).
+static int infer_by_levels(NrcHandle* h, cudaStream_t s, float* work, const float* in, uint32_t n, float* out) {
+    float* pos = work;
+    uint32_t* features = reinterpret_cast<uint32_t*>(work + 3 * static_cast<size_t>(kFeatureChunk));
+    const size_t chunks = (static_cast<size_t>(n) + kFeatureChunk - 1) / kFeatureChunk;
+    const size_t chunk = ((n + chunks - 1) / chunks + kTile - 1) / kTile * kTile;  // equal shares, whole tiles
+    for (size_t first = 0; first < n; first += chunk) {
+        const uint32_t m = static_cast<uint32_t>(std::min(n - first, chunk));
+        const float* q = in + first * 14;
+        grid_position_kernel<<<(m + 255) / 256, 256, 0, s>>>(q, m, pos);
+        grid_encode_kernel<<<std::max(h->num_sms, kGridLevels), kEncodeThreads, kEncodeSmem, s>>>(
+            h->ly, h->grid_words(false), pos, m, features, h->err);
+        NRC_CUDA(cudaGetLastError());
+        const int rc = launch_infer(h, s, features, true, q, nullptr, nullptr, m, out + first * 3);
+        if (rc) return rc;
+    }
     return NRC_OK;
 }
 
@@ -1166,31 +1363,18 @@ static int infer_impl(NrcHandle* h, void* stream, const float* in, const uint32_
     if (!h || !in || !out) return fail(NRC_ERR_INVALID_ARGUMENT, "nrc_infer: null argument");
     if (n == 0) return NRC_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int G = h->infer_groups;
-    const uint32_t tiles = (n + kTile - 1) / kTile;
-    const uint32_t grid = std::min<uint32_t>((tiles + G - 1) / G, static_cast<uint32_t>(h->num_sms));
-    const uint32_t smem = infer_smem(h->ly, G);
-    const bool vol = h->cfg.encoding == NRC_ENCODING_VOLUME;
-    const dim3 block(kTile * G);
-    const uint32_t* gw = h->grid_words(false);
-    if (G == 4) {
-        if (vol)
-            mlp_infer_kernel<144, 4, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
-        else
-            mlp_infer_kernel<64, 4, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
-    } else if (G == 2) {
-        if (vol)
-            mlp_infer_kernel<144, 2, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
-        else
-            mlp_infer_kernel<64, 2, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
-    } else {
-        if (vol)
-            mlp_infer_kernel<144, 1, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
-        else
-            mlp_infer_kernel<64, 1, kInferTmemActivations><<<grid, block, smem, s>>>(h->ly, h->blob_infer, gw, in, idx, dev_n, n, out, h->err);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (h->pool && !idx && !dev_n && n >= kFeatureMinQueries &&
+        cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        void* work = nullptr;
+        if (cudaMallocFromPoolAsync(&work, kFeatureBytes, h->pool, s) == cudaSuccess) {
+            const int rc = infer_by_levels(h, s, static_cast<float*>(work), in, n, out);
+            NRC_CUDA(cudaFreeAsync(work, s));
+            return rc;
+        }
+        cudaGetLastError();  // no room for the workspace: the fused kernel needs none
     }
-    NRC_CUDA(cudaGetLastError());
-    return NRC_OK;
+    return launch_infer(h, s, h->grid_words(false), false, in, idx, dev_n, n, out);
 }
 
 int nrc_infer(NrcHandle* h, void* stream, const float* in, uint32_t n, float* out) {
