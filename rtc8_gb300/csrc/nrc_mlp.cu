@@ -20,6 +20,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <memory>
+#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
@@ -191,11 +194,13 @@ __device__ __forceinline__ void one_blob8(float x, int b0, float (&v)[8]) {
 // NRC_ENCODING_VOLUME (144 features): sin and cos of pi 2^f x for the 3 position coordinates
 // (features 2(12a + f) and 2(12a + f) + 1), OneBlob(32) on vOut theta / pi and phi / 2 pi
 // (feature 72 + 32a + b), the local density (roughness slot) and the albedo (diffuse.r), 6 zeros.
+// HALF: 0 = the position's features, 1 = the rest (two threads per row), -1 = all.
+template <int HALF = -1>
 __device__ __forceinline__ void encode_row_volume(const float* q, uint8_t* tile, int r) {
     constexpr int K = 144;
     // Chunk k holds frequencies f0 .. f0 + 3 (f0 = 4 (k % 3)) of coordinate k / 3.
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
+    for (int k = 0; k < (HALF == 1 ? 0 : 9); ++k) {
         // sin / cos(pi v) with v = x 2^f0 exact: v = m + r (m integer, r in [0, 1)), so
         // sin(pi v) = (-1)^m sin(pi r) and likewise cos; the hardware approximation on [0, pi)
         // is accurate to ~4e-7. The next three frequencies follow by angle doubling,
@@ -219,6 +224,7 @@ __device__ __forceinline__ void encode_row_volume(const float* q, uint8_t* tile,
         }
         store8(tile, r, k, K, v);
     }
+    if constexpr (HALF == 0) return;
     const float theta = q[5] * (32.0f / 3.14159265f), phi = q[6] * (32.0f / 6.28318531f);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -272,35 +278,48 @@ __device__ __forceinline__ void grid_position(const float* q, float (&p)[3]) {
 // NRC_ENCODING_HASHGRID (64 features): levels 0..15 x 2 features from the FP16 tables (feature
 // 2 lv + f), then the reference encoding's OneBlob(4) on the 5 angle / roughness inputs
 // (32 + 4a + b) and identity on the 6 reflectance values (52..57), 6 zeros.
+// HALF: chunks (eight features) 0, 1, 4, 5 or 2, 3, 6, 7 (two threads per row), -1 = all. The training
+// kernel (HALF >= 0) runs few warps once per launch and fetches its instructions as it goes: it
+// keeps the chunk loop rolled.
+__device__ __forceinline__ void encode_grid_chunk(const NetLayout& ly, const uint32_t* __restrict__ grid, const float (&p)[3],
+                                                  uint8_t* tile, int r, int k) {
+    float v[8];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        uint32_t e[8];
+        float w[8];
+        grid_corners(ly, 4 * k + h, p, e, w);
+        uint32_t raw[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) raw[c] = __ldg(grid + e[c]);
+        float f0 = 0.0f, f1 = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&raw[c]));
+            f0 += w[c] * f.x;
+            f1 += w[c] * f.y;
+        }
+        v[2 * h] = f0;
+        v[2 * h + 1] = f1;
+    }
+    store8(tile, r, k, 64, v);
+}
+
+template <int HALF = -1>
 __device__ __forceinline__ void encode_row_hashgrid(const NetLayout& ly, const uint32_t* __restrict__ grid,
                                                     const float* q, uint8_t* tile, int r) {
     float p[3];
     grid_position(q, p);
+    if constexpr (HALF < 0) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float v[8];
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            uint32_t e[8];
-            float w[8];
-            grid_corners(ly, 4 * k + h, p, e, w);
-            uint32_t raw[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) raw[c] = __ldg(grid + e[c]);
-            float f0 = 0.0f, f1 = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&raw[c]));
-                f0 += w[c] * f.x;
-                f1 += w[c] * f.y;
-            }
-            v[2 * h] = f0;
-            v[2 * h + 1] = f1;
-        }
-        store8(tile, r, k, 64, v);
+        for (int k = 0; k < 4; ++k) encode_grid_chunk(ly, grid, p, tile, r, k);
+    } else {
+#pragma unroll 1
+        for (int k = 2 * HALF; k < 2 * HALF + 2; ++k) encode_grid_chunk(ly, grid, p, tile, r, k);
     }
 #pragma unroll
     for (int k = 4; k < 8; ++k) {
+        if (HALF >= 0 && (k - 4) / 2 != HALF) continue;
         float v[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = reference_feature(8 * k + i + 4, q);
@@ -308,15 +327,17 @@ __device__ __forceinline__ void encode_row_hashgrid(const NetLayout& ly, const u
     }
 }
 
-// The same input from features computed beforehand (grid_encode_kernel): f holds the 16 levels'
-// feature pairs, FP16.
-__device__ __forceinline__ void encode_row_features(const uint32_t (&f)[kGridLevels], const float* q, uint8_t* tile, int r) {
+// The same input from features computed beforehand (grid_encode_kernel): f holds the feature pairs
+// (FP16) of all 16 levels, or of levels 8 HALF .. 8 HALF + 7 (two threads per row).
+template <int HALF, int N>
+__device__ __forceinline__ void encode_row_features(const uint32_t (&f)[N], const float* q, uint8_t* tile, int r) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        *reinterpret_cast<uint4*>(tile + cm_offset(r, k * 8, 64)) =
+    for (int k = 0; k < N / 4; ++k)
+        *reinterpret_cast<uint4*>(tile + cm_offset(r, ((HALF == 1 ? 2 : 0) + k) * 8, 64)) =
             make_uint4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
 #pragma unroll
     for (int k = 4; k < 8; ++k) {
+        if (HALF >= 0 && (k - 4) / 2 != HALF) continue;
         float v[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = reference_feature(8 * k + i + 4, q);
@@ -324,19 +345,19 @@ __device__ __forceinline__ void encode_row_features(const uint32_t (&f)[kGridLev
     }
 }
 
-// Adds the gradient of the 32 hash-grid features of one query (`d`, loss-scaled) into the FP32
-// table gradient: corner c of level lv receives w_c x d[2 lv + f].
-__device__ __forceinline__ void grid_backward(const NetLayout& ly, const float* q, const float (&d)[32],
+// Adds the gradient of hash-grid levels lv0 .. lv0 + 7 of one query (`d`: their 16 features, loss-
+// scaled) into the FP32 table gradient: corner c of level lv receives w_c x d[2 (lv - lv0) + f].
+__device__ __forceinline__ void grid_backward(const NetLayout& ly, const float* q, int lv0, const float (&d)[16],
                                               float* __restrict__ grid_grad) {
     float p[3];
     grid_position(q, p);
 #pragma unroll 1
-    for (int lv = 0; lv < kGridLevels; ++lv) {
-        const float d0 = d[2 * lv], d1 = d[2 * lv + 1];
+    for (int k = 0; k < 8; ++k) {
+        const float d0 = d[2 * k], d1 = d[2 * k + 1];
         if (d0 == 0.0f && d1 == 0.0f) continue;
         uint32_t e[8];
         float w[8];
-        grid_corners(ly, lv, p, e, w);
+        grid_corners(ly, lv0 + k, p, e, w);
 #pragma unroll
         for (int c = 0; c < 8; ++c)
             atomicAdd(reinterpret_cast<float2*>(grid_grad) + e[c], make_float2(w[c] * d0, w[c] * d1));
@@ -344,21 +365,21 @@ __device__ __forceinline__ void grid_backward(const NetLayout& ly, const float* 
 }
 
 // Kernels specialised for the 144-wide volume input compile only its encoder.
-template <int IN>
+template <int IN, int HALF = -1>
 __device__ __forceinline__ void encode_row(const NetLayout& ly, const uint32_t* __restrict__ grid, const float* q,
                                            uint8_t* tile, int r) {
     if constexpr (IN == 144) {
-        encode_row_volume(q, tile, r);
+        encode_row_volume<HALF>(q, tile, r);
     } else if (ly.enc == NRC_ENCODING_REFERENCE) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = HALF == 1 ? 4 : 0; k < (HALF == 0 ? 4 : 8); ++k) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = reference_feature(8 * k + i, q);
             store8(tile, r, k, 64, v);
         }
     } else {
-        encode_row_hashgrid(ly, grid, q, tile, r);
+        encode_row_hashgrid<HALF>(ly, grid, q, tile, r);
     }
 }
 
@@ -458,6 +479,11 @@ __device__ __forceinline__ void load_row16(const uint8_t* tile, int r, int c0, i
 
 __host__ __device__ __forceinline__ uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
+// Programmatic dependent launch: a step's kernels start while the previous one drains and wait here
+// before their first access to global memory.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------ hash-grid features
 // Large inference batches compute the hash-grid features level by level: a CTA keeps ONE level's
 // table in shared memory (128 KB, brought in by one bulk copy) and takes a share of all positions
@@ -486,15 +512,25 @@ __global__ void __launch_bounds__(256) grid_position_kernel(const float* __restr
 // `table`. Corners, weights and sums as in grid_corners and encode_row_hashgrid (same order of
 // operations, so the same bits); the index arithmetic is in bytes (hash and mask shifted by two), one
 // three-input operation per hashed corner (172 -> 107 instructions per query and level).
-template <bool kHashed>
+// kRecords: the positions come from the query records (clamped here), otherwise from
+// grid_position_kernel's arrays.
+template <bool kHashed, bool kRecords>
 __device__ __forceinline__ void encode_level(const NetLayout& ly, uint32_t lv, uint32_t table, const float* __restrict__ pos,
                                              uint32_t first, uint32_t step, uint32_t n, uint32_t* __restrict__ out) {
     const float scale = ly.grid_scale[lv];
     const uint32_t res = ly.grid_res[lv], size = ly.grid_size[lv], mask = (size - 1u) << 2;
     float p[3] = {0.0f, 0.0f, 0.0f};
     auto load = [&](uint32_t i) {
+        if (i >= n) return;
+        if constexpr (kRecords) {
+            const float* q = pos + static_cast<size_t>(i) * 14;
+            const float2 xy = __ldg(reinterpret_cast<const float2*>(q));
+            const float v[3] = {xy.x, xy.y, __ldg(q + 2)};
+            grid_position(v, p);
+        } else {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) p[d] = i < n ? __ldg(pos + d * kFeatureChunk + i) : 0.0f;
+            for (int d = 0; d < 3; ++d) p[d] = __ldg(pos + d * kFeatureChunk + i);
+        }
     };
     load(first);
     for (uint32_t i = first; i < n; i += step) {
@@ -534,16 +570,19 @@ __device__ __forceinline__ void encode_level(const NetLayout& ly, uint32_t lv, u
     }
 }
 
-// features[level * kFeatureChunk + i] = the level's feature pair of position i (FP16), computed as
-// in encode_row_hashgrid. Bound by instruction issue and the shared-memory gathers.
+// features[level * stride + i] = the level's feature pair of position i (FP16), computed as in
+// encode_row_hashgrid. Bound by instruction issue and the shared-memory gathers.
+template <bool kRecords>
 __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const NetLayout ly, const uint32_t* __restrict__ grid,
                                                                         const float* __restrict__ pos, uint32_t n,
-                                                                        uint32_t* __restrict__ features,
+                                                                        uint32_t stride, uint32_t* __restrict__ features,
                                                                         unsigned int* __restrict__ err) {
     extern __shared__ __align__(128) uint32_t s_table[];
     __shared__ uint64_t s_bar;
     const uint32_t lv = blockIdx.x % kGridLevels, part = blockIdx.x / kGridLevels;
     const uint32_t parts = gridDim.x / kGridLevels + (lv < gridDim.x % kGridLevels ? 1u : 0u);
+    grid_launch_dependents();
+    grid_wait();
     if (threadIdx.x == 0) {
         mbar_init(&s_bar, 1);
         mbar_fence_init();
@@ -555,12 +594,12 @@ __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const Ne
         mbar_wait(&s_bar, 0);  // again bounded: the copy must not land in another CTA's shared memory
         return;
     }
-    uint32_t* const out = features + static_cast<size_t>(lv) * kFeatureChunk;
+    uint32_t* const out = features + static_cast<size_t>(lv) * stride;
     const uint32_t first = part * kEncodeThreads + threadIdx.x, step = parts * kEncodeThreads;
     if ((ly.grid_hashed >> lv) & 1u)
-        encode_level<true>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
+        encode_level<true, kRecords>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
     else
-        encode_level<false>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
+        encode_level<false, kRecords>(ly, lv, smem_u32(s_table), pos, first, step, n, out);
 }
 
 // ------------------------------------------------------------------------------ inference
@@ -629,7 +668,7 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
     for (uint32_t tile = blockIdx.x * G + g; tile < ntiles && ok; tile += stride) {
         const uint32_t row = tile * kTile + gt;
         if constexpr (FEAT)
-            encode_row_features(f, q, s_t, gt);
+            encode_row_features<-1>(f, q, s_t, gt);
         else
             encode_row<IN>(ly, grid, q, s_t, gt);
         // The next tile's queries load while this tile runs through the layers. (Encoding it
@@ -707,20 +746,36 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
 }
 
 // ------------------------------------------------------------------------------ training
-// One CTA per 128-sample tile: forward keeping all activations, relative-L2-luminance loss
-// gradient (denominator held constant), backward with weight gradients reduced into `grad`
-// (scaled by loss_scale) and the batch loss added to `loss`.
-// With the hash grid the backward pass also computes the first layer's input gradient and
-// scatters its 32 hash features into the table gradient (grad + ly.nparams).
+// One CTA of 256 threads per 128-sample tile, two threads (one of each warpgroup) per row: forward
+// keeping all activations, relative-L2-luminance loss gradient (denominator held constant),
+// backward with weight gradients reduced into `grad` (scaled by loss_scale) and the batch loss
+// added to `loss`. With the hash grid the backward pass also computes the first layer's input
+// gradient and scatters its 32 hash features into the table gradient (grad + ly.nparams).
+//
+// A tile is one chain of 2 L matrix products, each waiting for the epilogue before it: latency
+// bounds the kernel (128 tiles of a 16,384-record step on 152 SMs). So the epilogues are shared by
+// two warpgroups (half of the columns each), the weights arrive by one bulk copy while the rows are
+// encoded, and a layer's weight gradient (its product, then its reduction from tensor memory) is
+// taken off the chain: the next layer's products are issued first, into the other of two
+// accumulators.
+constexpr int kTrainThreads = 2 * kTile;
 template <int IN>
-__global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, const uint8_t* __restrict__ blob,
-                                                          const uint32_t* __restrict__ grid,
-                                                          const float* __restrict__ in, const float* __restrict__ target,
-                                                          uint32_t n, float* __restrict__ grad, float* __restrict__ loss,
-                                                          unsigned int* __restrict__ err) {
+constexpr uint32_t train_tmem_cols() { return IN == 144 ? 512 : 256; }  // 64 + 2 IN, a power of two
+
+// FEAT: the hash-grid features come from `grid` = grid_encode_kernel's (level * stride + row): the
+// gathers took 25,000 to 50,000 of the kernel's cycles (a 16,384-record step 52.9 -> 41 us).
+template <int IN, bool FEAT>
+__global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayout ly, const uint8_t* __restrict__ blob,
+                                                                  const uint32_t* __restrict__ grid,
+                                                                  const float* __restrict__ in,
+                                                                  const float* __restrict__ target, uint32_t n,
+                                                                  uint32_t stride, float* __restrict__ grad,
+                                                                  float* __restrict__ loss,
+                                                                  unsigned int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, wg = tid / kTile, r = tid % kTile, warp = r >> 5;
     const int L = ly.L;
+    const bool hash = IN == 64 && ly.enc == NRC_ENCODING_HASHGRID;
     uint8_t* s_w = smem;
     uint8_t* s_act0 = smem + align_up(ly.blob_bytes, 1024);
     uint8_t* s_acts = s_act0 + kTile * IN * 2;             // act_1 .. act_{L-1}, 16 KB each
@@ -728,30 +783,43 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, co
     uint8_t* s_dzb = s_dza + kTile * kWidth * 2;
     uint8_t* s_dzo = s_dzb + kTile * kWidth * 2;            // output gradient tile, 128 x 16
     uint8_t* s_slack = s_dzo + kTile * kOutPad * 2;         // absorbs MN-major over-reads
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_slack + 2048);
-    uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_bar + 1);
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_slack + 2048);  // chain products, weight gradients (2), weights
+    uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_bar + 4);
     auto act = [&](int j) -> uint8_t* { return j == 0 ? s_act0 : s_acts + (j - 1) * kTile * kWidth * 2; };
 
-    for (uint32_t i = tid; i < ly.blob_bytes / 16; i += kTile)
-        reinterpret_cast<uint4*>(s_w)[i] = __ldg(reinterpret_cast<const uint4*>(blob) + i);
-    for (uint32_t i = tid; i < 2048 / 16; i += kTile) reinterpret_cast<uint4*>(s_slack)[i] = make_uint4(0, 0, 0, 0);
-    if (warp == 0) tmem_alloc(s_slot, 256);
+    for (uint32_t i = tid; i < 2048 / 16; i += kTrainThreads) reinterpret_cast<uint4*>(s_slack)[i] = make_uint4(0, 0, 0, 0);
+    if (tid < 32) tmem_alloc(s_slot, train_tmem_cols<IN>());
     if (tid == 0) {
-        mbar_init(s_bar, 1);
+        for (int b = 0; b < 4; ++b) mbar_init(s_bar + b, 1);
         mbar_fence_init();
     }
-    const uint32_t row = blockIdx.x * kTile + tid;
+    grid_wait();
+    if (tid == 0) bulk_load(s_w, blob, ly.blob_bytes, s_bar + 3);
+    const uint32_t row = blockIdx.x * kTile + r;
     float q[14];
     load_query(in, nullptr, row, n, q);
-    encode_row<IN>(ly, grid, q, s_act0, tid);
+    if constexpr (FEAT) {
+        uint32_t f[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = row < n ? __ldg(grid + static_cast<size_t>(8 * wg + k) * stride + row) : 0u;
+        if (wg == 0)
+            encode_row_features<0>(f, q, s_act0, r);
+        else
+            encode_row_features<1>(f, q, s_act0, r);
+    } else if (wg == 0) {
+        encode_row<IN, 0>(ly, grid, q, s_act0, r);
+    } else {
+        encode_row<IN, 1>(ly, grid, q, s_act0, r);
+    }
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    bool ok = __syncthreads_and(tid != 0 || mbar_wait(s_bar + 3, 0));
     tc_fence_after();
+    // Not before this CTA holds its tensor memory: CTAs of the next step must not take it first.
+    grid_launch_dependents();
     const uint32_t tmem = *s_slot;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     uint32_t phase = 0;
-    bool ok = true;
 
     // ---- forward
     for (int j = 0; j < L && ok; ++j) {
@@ -765,14 +833,13 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, co
         tc_fence_after();
         if (!ok) break;
         if (j < L - 1) {
-#pragma unroll
-            for (int c = 0; c < kWidth / 16; ++c) {
-                float v[16];
-                tmem_ld16(tmem + lane_base + c * 16, v);
-                tmem_wait_ld();
-                store_row16_relu(act(j + 1), tid, c * 16, kWidth, v);
-            }
-        } else {
+            float v0[16], v1[16];
+            tmem_ld16(tmem + lane_base + wg * 32, v0);
+            tmem_ld16(tmem + lane_base + wg * 32 + 16, v1);
+            tmem_wait_ld();
+            store_row16_relu(act(j + 1), r, wg * 32, kWidth, v0);
+            store_row16_relu(act(j + 1), r, wg * 32 + 16, kWidth, v1);
+        } else if (wg == 0) {
             // output, loss and its gradient (rows beyond n contribute nothing)
             float v[16];
             tmem_ld16(tmem + lane_base, v);
@@ -800,7 +867,7 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, co
                     g[c] = gz * ly.loss_scale;
                 }
             }
-            store_row16(s_dzo, tid, 0, kOutPad, g);
+            store_row16(s_dzo, r, 0, kOutPad, g);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
             if ((tid & 31) == 0) atomicAdd(loss, l);
@@ -810,46 +877,77 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, co
         __syncthreads();
     }
 
-    // ---- backward: for matrix j, dW_j = dPre_{j+1}^T act_j and dPre_j = (dPre_{j+1} W_j) * relu'(act_j)
+    // ---- backward: for matrix j, dPre_j = (dPre_{j+1} W_j) * relu'(act_j) on the chain and
+    // dW_j = dPre_{j+1}^T act_j beside it (accumulator j & 1)
     uint8_t* dz = s_dzo;
     uint8_t* dz_next = s_dza;
-    const uint32_t tm_dx = tmem;        // columns [0, 64)
-    const uint32_t tm_dw = tmem + 64;   // columns [64, 64 + in_j)
-    for (int j = L - 1; j >= 0 && ok; --j) {
+    const uint32_t tm_dx = tmem;  // columns [0, 64)
+    auto tm_dw = [&](int j) -> uint32_t { return tmem + 64 + (j & 1) * IN; };
+    auto issue_backward = [&](int j) {
         const int K_out = ly.out[j], N_in = ly.in[j];
-        if (tid == 0) {
-            tc_fence_after();
-            // weight gradient: M = 128 (output features, rows beyond out_j unused), N = in_j, K = 128 samples
-            const uint32_t idw = idesc_f16(kTile, N_in, 1, 1);
-            const uint64_t adw = smem_desc(smem_u32(dz), static_cast<uint32_t>(K_out * 16), 128);
-            const uint64_t bdw = smem_desc(smem_u32(act(j)), static_cast<uint32_t>(N_in * 16), 128);
-#pragma unroll
-            for (int ks = 0; ks < kTile / 16; ++ks)  // 16 samples further: 2 K_out (2 N_in) in the address fields
-                mma_f16(tm_dw, adw + 2 * K_out * ks, bdw + 2 * N_in * ks, idw, ks > 0 ? 1u : 0u);
-            if (j > 0 || (IN == 64 && ly.enc == NRC_ENCODING_HASHGRID)) {
-                // input gradient: M = 128 samples, N = in_j, K = out_j; W_j read MN-major
-                const uint32_t idx = idesc_f16(kTile, N_in, 0, 1);
-                const uint64_t adx = smem_desc(smem_u32(dz), 128, static_cast<uint32_t>(K_out * 16));
-                const uint64_t bdx = smem_desc(smem_u32(s_w + ly.boff[j]), static_cast<uint32_t>(N_in * 16), 128);
-                for (int ks = 0; ks < K_out / 16; ++ks)
-                    mma_f16(tm_dx, adx + 16 * ks, bdx + 2 * N_in * ks, idx, ks > 0 ? 1u : 0u);
-            }
+        tc_fence_after();
+        if (j > 0 || hash) {
+            // input gradient: M = 128 samples, N = in_j, K = out_j; W_j read MN-major
+            const uint32_t idx = idesc_f16(kTile, N_in, 0, 1);
+            const uint64_t adx = smem_desc(smem_u32(dz), 128, static_cast<uint32_t>(K_out * 16));
+            const uint64_t bdx = smem_desc(smem_u32(s_w + ly.boff[j]), static_cast<uint32_t>(N_in * 16), 128);
+            for (int ks = 0; ks < K_out / 16; ++ks)
+                mma_f16(tm_dx, adx + 16 * ks, bdx + 2 * N_in * ks, idx, ks > 0 ? 1u : 0u);
             mma_commit(s_bar);
         }
-        ok = __syncthreads_and(mbar_wait(s_bar, phase));  // block-uniform decision
-        phase ^= 1;
-        tc_fence_after();
-        if (!ok) break;
+        // weight gradient: M = 128 (output features, rows beyond out_j unused), N = in_j, K = 128 samples
+        const uint32_t idw = idesc_f16(kTile, N_in, 1, 1);
+        const uint64_t adw = smem_desc(smem_u32(dz), static_cast<uint32_t>(K_out * 16), 128);
+        const uint64_t bdw = smem_desc(smem_u32(act(j)), static_cast<uint32_t>(N_in * 16), 128);
+#pragma unroll
+        for (int ks = 0; ks < kTile / 16; ++ks)  // 16 samples further: 2 K_out (2 N_in) in the address fields
+            mma_f16(tm_dw(j), adw + 2 * K_out * ks, bdw + 2 * N_in * ks, idw, ks > 0 ? 1u : 0u);
+        mma_commit(s_bar + 1 + (j & 1));
+    };
+    // The weight gradients' products complete one or two layers ahead of their reduction, so each
+    // accumulator has its own mbarrier (a wait on the parity of a phase must not miss the next one).
+    uint32_t phase_w = 0;  // bit b: accumulator b
+    if (ok && tid == 0) issue_backward(L - 1);
+    for (int j = L - 1; j >= 0 && ok; --j) {
+        const bool chain = j > 0 || hash;
+        if (chain) {
+            ok = __syncthreads_and(mbar_wait(s_bar, phase));  // block-uniform decision
+            phase ^= 1;
+            tc_fence_after();
+            if (!ok) break;
+        }
+        if (j > 0) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = wg * 32 + h * 16;
+                float v[16], a[16];
+                tmem_ld16(tm_dx + lane_base + c, v);
+                tmem_wait_ld();
+                load_row16(act(j), r, c, kWidth, a);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = a[i] > 0.0f ? v[i] : 0.0f;
+                store_row16(dz_next, r, c, kWidth, v);
+            }
+            dz = dz_next;
+            dz_next = dz_next == s_dza ? s_dzb : s_dza;
+            tc_fence_before();
+            fence_async_smem();
+            __syncthreads();
+            if (tid == 0) issue_backward(j - 1);
+        }
         // Weight-gradient rows: TMEM lane = output feature. The TMEM load is warp-collective, so
         // every lane of a warp that holds gradient rows takes part; only real rows are reduced.
-        const int out_real = j == L - 1 ? 3 : K_out;
-        if (warp * 32 < out_real) {
-            float* gdst = grad + ly.poff[j] + tid * N_in;
-            for (int c = 0; c < N_in / 16; ++c) {
+        const bool done = mbar_wait(s_bar + 1 + (j & 1), (phase_w >> (j & 1)) & 1u);
+        phase_w ^= 1u << (j & 1);
+        tc_fence_after();
+        const int out_real = j == L - 1 ? 3 : ly.out[j], N_in = ly.in[j];
+        if (warp * 32 < out_real && done) {
+            float* gdst = grad + ly.poff[j] + r * N_in;
+            for (int c = wg; c < N_in / 16; c += 2) {
                 float v[16];
-                tmem_ld16(tm_dw + lane_base + c * 16, v);
+                tmem_ld16(tm_dw(j) + lane_base + c * 16, v);
                 tmem_wait_ld();
-                if (tid < out_real) {
+                if (r < out_real) {
 #pragma unroll
                     for (int i = 0; i < 16; i += 4)
                         atomicAdd(reinterpret_cast<float4*>(gdst + c * 16 + i),
@@ -857,41 +955,21 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const NetLayout ly, co
                 }
             }
         }
-        if (j > 0) {
-#pragma unroll
-            for (int c = 0; c < kWidth / 16; ++c) {
-                float v[16], a[16];
-                tmem_ld16(tm_dx + lane_base + c * 16, v);
-                tmem_wait_ld();
-                load_row16(act(j), tid, c * 16, kWidth, a);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = a[i] > 0.0f ? v[i] : 0.0f;
-                store_row16(dz_next, tid, c * 16, kWidth, v);
-            }
-            dz = dz_next;
-            dz_next = dz_next == s_dza ? s_dzb : s_dza;
-        } else if (IN == 64 && ly.enc == NRC_ENCODING_HASHGRID) {
+        if (j == 0 && hash) {
             // gradient of the encoded input's hash features (columns 0..31) into the tables
-            float a[16], b[16], d[32];
-            tmem_ld16(tm_dx + lane_base, a);
-            tmem_ld16(tm_dx + lane_base + 16, b);
+            float d[16];
+            tmem_ld16(tm_dx + lane_base + wg * 16, d);
             tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                d[i] = a[i];
-                d[16 + i] = b[i];
-            }
-            if (row < n) grid_backward(ly, q, d, grad + ly.nparams);
+            if (row < n) grid_backward(ly, q, wg * 8, d, grad + ly.nparams);
         }
         tc_fence_before();
-        fence_async_smem();
-        __syncthreads();
+        if (!done) atomicOr(err, kErrTimeout);
     }
     if (!ok && tid == 0) atomicOr(err, kErrTimeout);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 256);
+    if (tid < 32) tmem_dealloc(tmem, train_tmem_cols<IN>());
 }
 
 // ------------------------------------------------------------------------------ elementwise kernels
@@ -925,56 +1003,99 @@ __global__ void pack_grid_kernel(const NetLayout ly, const float* __restrict__ w
 // beyond are hash-grid table entries (FP16 images grid_train / grid_infer); as published for the
 // multiresolution hash encoding (Mueller et al. 2022, section 4), they take no L2 term and an
 // entry whose gradient is exactly 0 skips its Adam step (its moments and value stay as they are).
-__global__ void adam_kernel(const NetLayout ly, float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ grad, float* __restrict__ ema, uint8_t* __restrict__ blob_train,
-                            uint8_t* __restrict__ blob_infer, __half* __restrict__ grid_train,
-                            __half* __restrict__ grid_infer, float lr, float beta1, float beta2, float eps, float l2,
-                            float inv_scale, float c1, float c2, float ema_decay, float ema_corr) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= ly.nparams + ly.grid_params) return;
-    if (p >= ly.nparams) {
-        float wi = w[p];
-        const float gr = grad[p];
-        if (gr != 0.0f) {
-            float g = gr * inv_scale;
-            float mi = beta1 * m[p] + (1.0f - beta1) * g;
-            float vi = beta2 * v[p] + (1.0f - beta2) * g * g;
-            m[p] = mi;
-            v[p] = vi;
-            wi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-            w[p] = wi;
-            grid_train[p - ly.nparams] = __float2half_rn(wi);
+// The gradient and loss accumulators are moved to `grad_out` and `loss_out` (what the caller can
+// read) and cleared for the next step, which so needs no launch to clear them.
+struct Adam {
+    float *w, *m, *v, *grad, *grad_out, *loss, *loss_out, *ema;
+    uint8_t *blob_train, *blob_infer;
+    __half *grid_train, *grid_infer;
+    float lr, beta1, beta2, eps, l2, inv_scale, c1, c2, ema_decay, ema_corr;
+};
+
+// Four consecutive table features, feature e of the tables on, with gradients g4.
+__device__ __forceinline__ void adam_table4(const NetLayout& ly, const Adam& a, int e, float4 g4) {
+    const int p = ly.nparams + e;
+    float4 w4 = *reinterpret_cast<const float4*>(a.w + p);
+    float* wi = reinterpret_cast<float*>(&w4);
+    const float* gr = reinterpret_cast<const float*>(&g4);
+    if (gr[0] != 0.0f || gr[1] != 0.0f || gr[2] != 0.0f || gr[3] != 0.0f) {
+        float4 m4 = *reinterpret_cast<const float4*>(a.m + p), v4 = *reinterpret_cast<const float4*>(a.v + p);
+        float* mi = reinterpret_cast<float*>(&m4);
+        float* vi = reinterpret_cast<float*>(&v4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (gr[i] == 0.0f) continue;
+            const float g = gr[i] * a.inv_scale;
+            mi[i] = a.beta1 * mi[i] + (1.0f - a.beta1) * g;
+            vi[i] = a.beta2 * vi[i] + (1.0f - a.beta2) * g * g;
+            wi[i] -= a.lr * (mi[i] / a.c1) / (sqrtf(vi[i] / a.c2) + a.eps);
         }
-        float wi_inf = wi;
-        if (ema_decay > 0.0f) {
-            float e = ema_decay * ema[p] + (1.0f - ema_decay) * wi;
-            ema[p] = e;
-            wi_inf = e / ema_corr;
-        }
-        grid_infer[p - ly.nparams] = __float2half_rn(wi_inf);
-        return;
+        *reinterpret_cast<float4*>(a.m + p) = m4;
+        *reinterpret_cast<float4*>(a.v + p) = v4;
+        *reinterpret_cast<float4*>(a.w + p) = w4;
+        *reinterpret_cast<uint2*>(a.grid_train + e) = make_uint2(pack_half2(wi[0], wi[1]), pack_half2(wi[2], wi[3]));
     }
+    *reinterpret_cast<float4*>(a.grad_out + p) = g4;
+    if (a.ema_decay > 0.0f) {
+        float4 e4 = *reinterpret_cast<const float4*>(a.ema + p);
+        float* ei = reinterpret_cast<float*>(&e4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            ei[i] = a.ema_decay * ei[i] + (1.0f - a.ema_decay) * wi[i];
+            wi[i] = ei[i] / a.ema_corr;
+        }
+        *reinterpret_cast<float4*>(a.ema + p) = e4;
+    }
+    *reinterpret_cast<uint2*>(a.grid_infer + e) = make_uint2(pack_half2(wi[0], wi[1]), pack_half2(wi[2], wi[3]));
+}
+
+// One matrix weight.
+__device__ __forceinline__ void adam_weight(const NetLayout& ly, const Adam& a, int p) {
+    const float gr = a.grad[p];
+    a.grad[p] = 0.0f;
+    a.grad_out[p] = gr;
     ParamIndex x = param_index(ly, p);
     bool real = x.i < (x.j == 0 ? ly.in_real : ly.in[x.j]) && x.o < (x.j == ly.L - 1 ? 3 : ly.out[x.j]);
-    float wi = w[p];
+    float wi = a.w[p];
     if (real) {
-        float g = grad[p] * inv_scale + l2 * wi;
-        float mi = beta1 * m[p] + (1.0f - beta1) * g;
-        float vi = beta2 * v[p] + (1.0f - beta2) * g * g;
-        m[p] = mi;
-        v[p] = vi;
-        wi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[p] = wi;
+        float g = gr * a.inv_scale + a.l2 * wi;
+        float mi = a.beta1 * a.m[p] + (1.0f - a.beta1) * g;
+        float vi = a.beta2 * a.v[p] + (1.0f - a.beta2) * g * g;
+        a.m[p] = mi;
+        a.v[p] = vi;
+        wi -= a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+        a.w[p] = wi;
     }
     uint32_t off = cm_offset(x.o, x.i, ly.in[x.j]);
-    *reinterpret_cast<__half*>(blob_train + ly.boff[x.j] + off) = __float2half_rn(wi);
+    *reinterpret_cast<__half*>(a.blob_train + ly.boff[x.j] + off) = __float2half_rn(wi);
     float wi_inf = wi;
-    if (ema_decay > 0.0f) {
-        float e = ema_decay * ema[p] + (1.0f - ema_decay) * wi;
-        ema[p] = e;
-        wi_inf = e / ema_corr;
+    if (a.ema_decay > 0.0f) {
+        float e = a.ema_decay * a.ema[p] + (1.0f - a.ema_decay) * wi;
+        a.ema[p] = e;
+        wi_inf = e / a.ema_corr;
     }
-    *reinterpret_cast<__half*>(blob_infer + ly.boff[x.j] + off) = __float2half_rn(wi_inf);
+    *reinterpret_cast<__half*>(a.blob_infer + ly.boff[x.j] + off) = __float2half_rn(wi_inf);
+}
+
+__global__ void __launch_bounds__(256) adam_kernel(const NetLayout ly, const Adam a) {
+    grid_launch_dependents();
+    grid_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.loss_out = *a.loss;
+        *a.loss = 0.0f;
+    }
+    const int mlp_blocks = (ly.nparams + 255) / 256;
+    if (static_cast<int>(blockIdx.x) < mlp_blocks) {
+        const int p = blockIdx.x * 256 + threadIdx.x;
+        if (p < ly.nparams) adam_weight(ly, a, p);
+        return;
+    }
+    const int e = (static_cast<int>(blockIdx.x) - mlp_blocks) * 1024 + threadIdx.x * 4;
+    if (e >= ly.grid_params) return;
+    float4* g = reinterpret_cast<float4*>(a.grad + ly.nparams + e);
+    const float4 g4 = *g;
+    if (g4.x != 0.0f || g4.y != 0.0f || g4.z != 0.0f || g4.w != 0.0f) *g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    adam_table4(ly, a, e, g4);
 }
 
 template <int IN>
@@ -1128,10 +1249,14 @@ const void* infer_kernel_ptr(int enc, int groups, bool features) {
                        : (groups == 2 ? infer_kernel_for<2>(enc, features) : infer_kernel_for<1>(enc, features));
 }
 constexpr uint32_t kEncodeSmem = kGridMaxEntries * 4;
+// Training steps of so many records take their features from grid_encode_kernel too (us per step, in
+// the training kernel against this: 1,024 records 54 / 28, 4,096 61 / 34, 16,384 59 / 45); larger ones
+// would need a larger buffer beside every cache.
+constexpr uint32_t kTrainLevelsMin = 256, kTrainLevelsMax = 1u << 18;
 constexpr size_t kFeatureBytes = static_cast<size_t>(kFeatureChunk) * (3 + kGridLevels) * 4;
 uint32_t train_smem(const NetLayout& l) {
     return align_up(l.blob_bytes, 1024) + kTile * l.in_dim * 2 + (l.L - 1) * kTile * kWidth * 2 +
-           2 * kTile * kWidth * 2 + kTile * kOutPad * 2 + 2048 + 16;
+           2 * kTile * kWidth * 2 + kTile * kOutPad * 2 + 2048 + 48;
 }
 
 }  // namespace
@@ -1139,18 +1264,30 @@ uint32_t train_smem(const NetLayout& l) {
 
 using namespace nrc;
 
+// Workspaces of large hash-grid batches (grid_encode_kernel), taken and given back in stream order, so
+// that calls on several streams each have their own. One pool per device, shared by the caches that
+// are alive and given back with the last of them; it keeps as many workspaces (80 MB each) as were in
+// use at once.
+struct WorkspacePool {
+    cudaMemPool_t pool = nullptr;
+    ~WorkspacePool() {
+        if (pool) cudaMemPoolDestroy(pool);
+    }
+};
+
 struct NrcHandle {
     NrcConfig cfg;
     NetLayout ly;
     int num_sms = 0;
     int infer_groups = 1;  // 128-row tiles in flight per inference CTA
-    float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *ema = nullptr, *loss = nullptr;
+    float *w = nullptr, *m = nullptr, *v = nullptr, *ema = nullptr;
+    float *grad = nullptr, *loss = nullptr;          // accumulators of a step, zero between steps
+    float *grad_out = nullptr, *loss_out = nullptr;  // the last step's
     uint8_t *blob_train = nullptr, *blob_infer = nullptr;
     __half *grid_train = nullptr, *grid_infer = nullptr;  // FP16 hash-grid tables (hash grid only)
     unsigned int* err = nullptr;
-    // Workspaces of large hash-grid inference batches: taken and given back in stream order, so that
-    // calls on several streams each have their own.
-    cudaMemPool_t pool = nullptr;
+    uint32_t* train_features = nullptr;      // hash grid only: features of a training step's records
+    std::shared_ptr<WorkspacePool> pool;  // hash grid only; null = batches run the fused kernels
     uint64_t steps = 0;
     int total_params() const { return ly.nparams + ly.grid_params; }
     const uint32_t* grid_words(bool train) const {
@@ -1164,6 +1301,48 @@ int alloc(T** p, size_t n) {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), n * sizeof(T));
     if (e != cudaSuccess) return fail(NRC_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     return NRC_OK;
+}
+
+// Uniform initialisation with bound sqrt(6 / (fan_in + fan_out)); padded rows/columns are 0.
+// Hash-grid entries start uniform in [-1e-4, 1e-4] (the published initialisation).
+std::vector<float> initial_weights(const NetLayout& ly, int total, uint32_t seed) {
+    std::vector<float> w(total, 0.0f);
+    std::mt19937 gen(seed);
+    for (int j = 0; j < ly.L; ++j) {
+        const int in_real = j == 0 ? ly.in_real : ly.in[j];
+        const int out_real = j == ly.L - 1 ? 3 : ly.out[j];
+        const float bound = std::sqrt(6.0f / static_cast<float>(in_real + out_real));
+        std::uniform_real_distribution<float> u(-bound, bound);
+        for (int o = 0; o < out_real; ++o)
+            for (int i = 0; i < in_real; ++i) w[ly.poff[j] + o * ly.in[j] + i] = u(gen);
+    }
+    std::uniform_real_distribution<float> ug(-1e-4f, 1e-4f);
+    for (int p = ly.nparams; p < total; ++p) w[p] = ug(gen);
+    return w;
+}
+
+// The device's workspace pool, with one workspace reserved; null where there is no room for it.
+std::shared_ptr<WorkspacePool> workspace_pool(int device) {
+    static std::mutex mutex;
+    static std::map<int, std::weak_ptr<WorkspacePool>> pools;
+    std::lock_guard<std::mutex> lock(mutex);
+    std::shared_ptr<WorkspacePool> p = pools[device].lock();
+    if (p) return p;
+    p = std::make_shared<WorkspacePool>();
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = UINT64_MAX;
+    void* work = nullptr;
+    if (cudaMemPoolCreate(&p->pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+        cudaMallocFromPoolAsync(&work, kFeatureBytes, p->pool, 0) != cudaSuccess || cudaFreeAsync(work, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    pools[device] = p;
+    return p;
 }
 
 int set_kernel_smem(const void* k, uint32_t bytes) {
@@ -1237,29 +1416,17 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     const int ng = std::max(h->ly.grid_params, 2);
     int rc;
     if ((rc = alloc(&h->w, np)) || (rc = alloc(&h->m, np)) || (rc = alloc(&h->v, np)) || (rc = alloc(&h->grad, np)) ||
-        (rc = alloc(&h->ema, np)) || (rc = alloc(&h->loss, 1)) || (rc = alloc(&h->blob_train, h->ly.blob_bytes)) ||
+        (rc = alloc(&h->grad_out, np)) || (rc = alloc(&h->loss_out, 1)) || (rc = alloc(&h->ema, np)) || (rc = alloc(&h->loss, 1)) || (rc = alloc(&h->blob_train, h->ly.blob_bytes)) ||
         (rc = alloc(&h->blob_infer, h->ly.blob_bytes)) || (rc = alloc(&h->grid_train, ng)) ||
         (rc = alloc(&h->grid_infer, ng)) || (rc = alloc(&h->err, 1))) {
         nrc_destroy(h);
         return rc;
     }
-    // Uniform initialisation with bound sqrt(6 / (fan_in + fan_out)); padded rows/columns are 0.
-    std::vector<float> w(np, 0.0f);
-    std::mt19937 gen(cfg->seed);
-    for (int j = 0; j < h->ly.L; ++j) {
-        int in_real = j == 0 ? h->ly.in_real : h->ly.in[j];
-        int out_real = j == h->ly.L - 1 ? 3 : h->ly.out[j];
-        float bound = std::sqrt(6.0f / static_cast<float>(in_real + out_real));
-        std::uniform_real_distribution<float> u(-bound, bound);
-        for (int o = 0; o < out_real; ++o)
-            for (int i = 0; i < in_real; ++i) w[h->ly.poff[j] + o * h->ly.in[j] + i] = u(gen);
-    }
-    // Hash-grid entries start uniform in [-1e-4, 1e-4] (the published initialisation).
-    std::uniform_real_distribution<float> ug(-1e-4f, 1e-4f);
-    for (int p = h->ly.nparams; p < np; ++p) w[p] = ug(gen);
+    const std::vector<float> w = initial_weights(h->ly, np, cfg->seed);
     if (cudaMemcpy(h->w, w.data(), np * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(h->m, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->v, 0, np * sizeof(float)) != cudaSuccess ||
         cudaMemset(h->grad, 0, np * sizeof(float)) != cudaSuccess ||
+        cudaMemset(h->grad_out, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->loss, 0, sizeof(float)) != cudaSuccess ||
         cudaMemset(h->ema, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->err, 0, sizeof(unsigned int)) != cudaSuccess) {
         nrc_destroy(h);
         return fail(NRC_ERR_CUDA, "nrc_create: initial upload failed");
@@ -1273,8 +1440,8 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     const bool vol = cfg->encoding == NRC_ENCODING_VOLUME;
     h->infer_groups = infer_groups(h->ly);
     if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, false), infer_smem(h->ly, h->infer_groups))) ||
-        (rc = set_kernel_smem(vol ? reinterpret_cast<const void*>(mlp_train_kernel<144>)
-                                  : reinterpret_cast<const void*>(mlp_train_kernel<64>),
+        (rc = set_kernel_smem(vol ? reinterpret_cast<const void*>(mlp_train_kernel<144, false>)
+                                  : reinterpret_cast<const void*>(mlp_train_kernel<64, false>),
                               train_smem(h->ly)))) {
         nrc_destroy(h);
         return rc;
@@ -1282,23 +1449,17 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     if (cfg->encoding == NRC_ENCODING_HASHGRID) {
         if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, true),
                                   infer_smem(h->ly, h->infer_groups))) ||
-            (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel), kEncodeSmem))) {
+            (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel<false>), kEncodeSmem)) ||
+            (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel<true>), kEncodeSmem)) ||
+            (rc = set_kernel_smem(reinterpret_cast<const void*>(mlp_train_kernel<64, true>), train_smem(h->ly)))) {
             nrc_destroy(h);
             return rc;
         }
-        // The pool keeps its memory between calls; the first workspace is reserved here. Without it
-        // (little memory left) large batches run the fused kernel.
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        uint64_t keep = UINT64_MAX;
-        void* work = nullptr;
-        if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
-            cudaMallocFromPoolAsync(&work, kFeatureBytes, h->pool, 0) != cudaSuccess ||
-            cudaFreeAsync(work, 0) != cudaSuccess)
-            cudaGetLastError();
+        if ((rc = alloc(&h->train_features, static_cast<size_t>(kGridLevels) * kTrainLevelsMax))) {
+            nrc_destroy(h);
+            return rc;
+        }
+        h->pool = workspace_pool(dev);
     }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         nrc_destroy(h);
@@ -1316,14 +1477,24 @@ int nrc_destroy(NrcHandle* h) {
     cudaFree(h->grad);
     cudaFree(h->ema);
     cudaFree(h->loss);
+    cudaFree(h->grad_out);
+    cudaFree(h->loss_out);
+    cudaFree(h->train_features);
     cudaFree(h->blob_train);
     cudaFree(h->blob_infer);
     cudaFree(h->grid_train);
     cudaFree(h->grid_infer);
     cudaFree(h->err);
-    if (h->pool) cudaMemPoolDestroy(h->pool);
     delete h;
     return NRC_OK;
+}
+
+// Whether a batch of n records goes through the hash grid level by level (needs a workspace, which a
+// captured stream does not take).
+static bool by_levels(NrcHandle* h, cudaStream_t s, uint32_t n) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    return h->pool && n >= kFeatureMinQueries && cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
+           capture == cudaStreamCaptureStatusNone;
 }
 
 static int launch_infer(NrcHandle* h, cudaStream_t s, const uint32_t* grid_or_features, bool features, const float* in,
@@ -1349,8 +1520,8 @@ static int infer_by_levels(NrcHandle* h, cudaStream_t s, float* work, const floa
         const uint32_t m = static_cast<uint32_t>(std::min(n - first, chunk));
         const float* q = in + first * 14;
         grid_position_kernel<<<(m + 255) / 256, 256, 0, s>>>(q, m, pos);
-        grid_encode_kernel<<<std::max(h->num_sms, kGridLevels), kEncodeThreads, kEncodeSmem, s>>>(
-            h->ly, h->grid_words(false), pos, m, features, h->err);
+        grid_encode_kernel<false><<<std::max(h->num_sms, kGridLevels), kEncodeThreads, kEncodeSmem, s>>>(
+            h->ly, h->grid_words(false), pos, m, kFeatureChunk, features, h->err);
         NRC_CUDA(cudaGetLastError());
         const int rc = launch_infer(h, s, features, true, q, nullptr, nullptr, m, out + first * 3);
         if (rc) return rc;
@@ -1363,11 +1534,9 @@ static int infer_impl(NrcHandle* h, void* stream, const float* in, const uint32_
     if (!h || !in || !out) return fail(NRC_ERR_INVALID_ARGUMENT, "nrc_infer: null argument");
     if (n == 0) return NRC_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (h->pool && !idx && !dev_n && n >= kFeatureMinQueries &&
-        cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    if (!idx && !dev_n && by_levels(h, s, n)) {
         void* work = nullptr;
-        if (cudaMallocFromPoolAsync(&work, kFeatureBytes, h->pool, s) == cudaSuccess) {
+        if (cudaMallocFromPoolAsync(&work, kFeatureBytes, h->pool->pool, s) == cudaSuccess) {
             const int rc = infer_by_levels(h, s, static_cast<float*>(work), in, n, out);
             NRC_CUDA(cudaFreeAsync(work, s));
             return rc;
@@ -1398,29 +1567,48 @@ int nrc_train(NrcHandle* h, void* stream, const float* in, const float* target, 
     if (n == 0) return NRC_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const NetLayout& ly = h->ly;
-    const int np = h->total_params();
-    NRC_CUDA(cudaMemsetAsync(h->grad, 0, np * sizeof(float), s));
-    NRC_CUDA(cudaMemsetAsync(h->loss, 0, sizeof(float), s));
-    uint32_t tiles = (n + kTile - 1) / kTile;
-    uint32_t smem = train_smem(ly);
-    const uint32_t* gw = h->grid_words(true);
-    if (h->cfg.encoding == NRC_ENCODING_VOLUME)
-        mlp_train_kernel<144><<<tiles, kTile, smem, s>>>(ly, h->blob_train, gw, in, target, n, h->grad, h->loss, h->err);
-    else
-        mlp_train_kernel<64><<<tiles, kTile, smem, s>>>(ly, h->blob_train, gw, in, target, n, h->grad, h->loss, h->err);
+    const uint32_t tiles = (n + kTile - 1) / kTile;
     ++h->steps;
     const NrcConfig& c = h->cfg;
-    float c1 = 1.0f - std::pow(c.beta1, static_cast<float>(h->steps));
-    float c2 = 1.0f - std::pow(c.beta2, static_cast<float>(h->steps));
+    const float c1 = 1.0f - std::pow(c.beta1, static_cast<float>(h->steps));
+    const float c2 = 1.0f - std::pow(c.beta2, static_cast<float>(h->steps));
     // The EMA starts from the initial weights (not from zero), so it needs no bias correction.
-    const float ema_corr = 1.0f;
-    adam_kernel<<<(np + 255) / 256, 256, 0, s>>>(ly, h->w, h->m, h->v, h->grad, h->ema, h->blob_train, h->blob_infer,
-                                                 h->grid_train, h->grid_infer, c.learning_rate, c.beta1, c.beta2,
-                                                 c.epsilon, c.l2_reg, 1.0f / c.loss_scale, c1, c2, c.ema_decay,
-                                                 ema_corr);
-    NRC_CUDA(cudaGetLastError());
+    const Adam adam{h->w, h->m, h->v, h->grad, h->grad_out, h->loss, h->loss_out, h->ema, h->blob_train, h->blob_infer,
+                    h->grid_train, h->grid_infer, c.learning_rate, c.beta1, c.beta2, c.epsilon, c.l2_reg,
+                    1.0f / c.loss_scale, c1, c2, c.ema_decay, 1.0f};
+    // A step's kernels start while their predecessor on the stream drains (they wait for it before
+    // their first access to memory).
+    cudaLaunchAttribute overlap{};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.stream = s;
+    lc.attrs = &overlap;
+    lc.numAttrs = 1;
+    auto shape = [&](uint32_t grid, uint32_t block, uint32_t smem) {
+        lc.gridDim = dim3(grid);
+        lc.blockDim = dim3(block);
+        lc.dynamicSmemBytes = smem;
+        return &lc;
+    };
+    const uint8_t* blob = h->blob_train;
+    const uint32_t* gw = h->grid_words(true);
+    if (c.encoding == NRC_ENCODING_HASHGRID && n >= kTrainLevelsMin && n <= kTrainLevelsMax) {
+        uint32_t* features = h->train_features;
+        const uint32_t stride = tiles * kTile;
+        NRC_CUDA(cudaLaunchKernelEx(shape(std::max(h->num_sms, kGridLevels), kEncodeThreads, kEncodeSmem),
+                                    grid_encode_kernel<true>, ly, gw, in, n, stride, features, h->err));
+        NRC_CUDA(cudaLaunchKernelEx(shape(tiles, kTrainThreads, train_smem(ly)), mlp_train_kernel<64, true>, ly, blob,
+                                    static_cast<const uint32_t*>(features), in, target, n, stride, h->grad, h->loss, h->err));
+    } else {
+        NRC_CUDA(cudaLaunchKernelEx(shape(tiles, kTrainThreads, train_smem(ly)),
+                                    c.encoding == NRC_ENCODING_VOLUME ? mlp_train_kernel<144, false> : mlp_train_kernel<64, false>,
+                                    ly, blob, gw, in, target, n, 0u, h->grad, h->loss, h->err));
+    }
+    NRC_CUDA(cudaLaunchKernelEx(shape((ly.nparams + 255) / 256 + (ly.grid_params + 1023) / 1024, 256, 0), adam_kernel, ly,
+                                adam));
     if (loss_out) {
-        NRC_CUDA(cudaMemcpyAsync(loss_out, h->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+        NRC_CUDA(cudaMemcpyAsync(loss_out, h->loss_out, sizeof(float), cudaMemcpyDeviceToHost, s));
         NRC_CUDA(cudaStreamSynchronize(s));
     }
     return NRC_OK;
@@ -1458,7 +1646,7 @@ int nrc_set_params(NrcHandle* h, const float* host) {
 int nrc_get_gradients(NrcHandle* h, float* host) {
     if (!h || !host) return fail(NRC_ERR_INVALID_ARGUMENT, "null argument");
     NRC_CUDA(cudaDeviceSynchronize());
-    NRC_CUDA(cudaMemcpy(host, h->grad, h->total_params() * sizeof(float), cudaMemcpyDeviceToHost));
+    NRC_CUDA(cudaMemcpy(host, h->grad_out, h->total_params() * sizeof(float), cudaMemcpyDeviceToHost));
     const float inv = 1.0f / h->cfg.loss_scale;
     for (int i = 0; i < h->total_params(); ++i) host[i] *= inv;
     return NRC_OK;

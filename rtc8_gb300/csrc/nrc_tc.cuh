@@ -144,9 +144,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after `limit` polls (each poll may suspend the thread briefly) and
-// returns false, so a kernel can record an error and leave instead of hanging.
-__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t limit = 1u << 24) {
+// Bounded wait: gives up after `limit` polls (a poll suspends the thread for up to 4 us: about a
+// second) and returns false, so a kernel can record an error and leave instead of hanging.
+__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t limit = 1u << 18) {
     for (uint32_t i = 0; i < limit; ++i)
         if (mbar_try_wait(mbar, parity)) return true;
     return false;
