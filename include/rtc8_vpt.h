@@ -240,9 +240,9 @@ typedef struct VptSurfaceInstance {
  * of the emitting triangles (per triangle luminance(emittance) x object-space area, per
  * geometry instance, per instance the group's total x scale^2: compute_light_probs.cu:19-137,
  * renderer_scene.cpp:353-468) and widens the world box (compute_light_probs.cu:139-157).
- * Plain launches of a context with surfaces run the surface tracer (reference and
- * configuration modes, either stream layout; not the wavefront tracer, not leaf staging, not
- * the radiance-cache passes). With surfaces a volume is optional (vpt_clear_volume). */
+ * Launches of a context with surfaces (plain ones in either mode and stream layout, and the
+ * radiance-cache passes) run the tracker with work queues, also where the wavefront tracker or
+ * leaf staging is chosen. With surfaces a volume is optional (vpt_clear_volume). */
 int vpt_set_surfaces(VptContext* ctx, const VptSurfaceMaterial* materials, uint32_t num_materials,
                      const VptSurfaceGeometry* geometries, uint32_t num_geometries,
                      const VptSurfaceInstance* instances, uint32_t num_instances);
@@ -392,11 +392,11 @@ int vpt_set_tracker(VptContext* ctx, int32_t kind, int32_t slots_per_sm, int32_t
  * default). Decisions and values are those of the unstaged tracker. */
 int vpt_set_leaf_staging(VptContext* ctx, int32_t min_lanes);
 /* Launch shape of the persistent trackers: CTAs per SM, threads per CTA (a multiple of 32 up to
- * 128), and the number of parked lanes of a warp that triggers its joint event phase (scenes with
- * meshes and leaf staging only: the tracker of volume scenes has work queues instead); 0 = defaults:
- * three CTAs of 256 threads per SM for volume scenes, as many 128-thread CTAs as fit for the other
- * forms. Contexts whose launches run concurrently on one GPU (several scenes at once) do better with
- * 128-thread CTAs, which can share an SM. */
+ * 128), and, with leaf staging only, the number of parked lanes of a warp that triggers its joint
+ * event phase (the default tracker has work queues instead); 0 = defaults: three CTAs of 256 threads
+ * per SM, with leaf staging as many of 128 as fit and 16 parked lanes. Contexts whose launches run
+ * concurrently on one GPU (several scenes at once) do better with 128-thread CTAs, which can share
+ * an SM. */
 int vpt_set_launch_shape(VptContext* ctx, int32_t ctas_per_sm, int32_t threads_per_cta,
                          int32_t park_threshold);
 

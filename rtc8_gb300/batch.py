@@ -22,9 +22,7 @@ from .configs import C1, SceneConfig, VolumeSpec
 from .renderer import Renderer, setup_scene
 
 # Launch shapes the autotuner tries: (CTAs per SM, park threshold); 0 = the defaults. The batch's
-# launches run CTAs of 128 threads (BATCH_THREADS): alone, a scene's plain launch is fastest as one
-# 896-thread CTA per SM, but the batch's concurrent launches then cannot share an SM (16 scenes:
-# 606 M paths/s against 647 M with 128-thread CTAs).
+# launches run CTAs of 128 threads (BATCH_THREADS), so that concurrent launches share an SM.
 LAUNCH_CANDIDATES = [(0, 0), (0, 16), (0, 28), (6, 24), (5, 24)]
 BATCH_THREADS = 128
 

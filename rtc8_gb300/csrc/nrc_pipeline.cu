@@ -223,20 +223,8 @@ int launch_pass(VptContext* c, cudaStream_t s, int mode, uint32_t buf, uint32_t 
     tp.nrc_train_termination = c->nrc_train_termination;
     NRCP_CUDA(cudaMemsetAsync(c->d_work, 0, sizeof(unsigned int), s));
     const bool grid_maj = c->has_volume && c->frame.majorant_mode == 1;
-    if (c->surf) {
-        const int threads = c->threads > 0 ? c->threads : 128;
-        size_t smem = 0;
-        if (grid_maj && c->mx * c->my * c->mz <= vpt::kMajSmemCells) {
-            tp.maj_in_smem = 1;
-            smem = static_cast<size_t>(c->mx) * c->my * c->mz * sizeof(float);
-        }
-        const void* kernel = vpt::nrc_surface_kernel_ptr(mode, grid_maj, tp.grid.st_values != nullptr);
-        const int ctas = vpt::persistent_grid(c, threads, kernel, smem);
-        vpt::launch_nrc_surfaces(tp, mode, grid_maj, ctas, threads, smem, s);
-    } else {
-        NRCP_CUDA(vpt::launch_queues(tp, mode, grid_maj, c->threads > 0 ? c->threads : vpt::kQueueThreads,
-                                     c->ctas_per_sm, c->num_sms, s));
-    }
+    NRCP_CUDA(vpt::launch_queues(tp, mode, grid_maj, c->threads > 0 ? c->threads : vpt::kQueueThreads, c->ctas_per_sm,
+                                 c->num_sms, s));
     NRCP_CUDA(cudaGetLastError());
     if (stream_mode == 1 && spp > 0) {
         vpt::launch_frame_update(c->d_frame, spp, false, 0, s);

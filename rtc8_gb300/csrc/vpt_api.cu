@@ -530,10 +530,7 @@ int fill_trace_params(VptContextImpl* c, TraceParams* tp) {
     }
     g.global_majorant = c->global_majorant;
     g.st_table = c->d_st_table;
-    // Scenes whose few triangles are tested in a flat loop keep the leaves: that kernel is bound by
-    // instruction fetch and took 25.0 ms with the stencils against 23.7 ms (512^2 x 4 spp, 36
-    // triangles); through the BVH the stencils win, 30.3 against 35.3 ms.
-    g.st_values = c->surf && c->surf->num_tris <= kFlatTriangles ? nullptr : c->d_st_values;
+    g.st_values = c->d_st_values;
     g.sx = c->lx + 1;
     g.sy = c->ly + 1;
     g.sz = c->lz + 1;
@@ -626,15 +623,9 @@ static int launch_plain_impl(VptContext* c, void* stream, uint32_t spp, uint32_t
     // Leaf staging: majorant-grid tracker on sample-parallel streams (and its logged form).
     const bool stage = c->leaf_stage_min > 0 && grid_maj && (dlog != nullptr || tp.stream_mode == 1) && !c->surf;
     tp.leaf_stage_min = stage ? c->leaf_stage_min : 0;
-    const int threads = c->threads > 0 ? c->threads : 128;  // of the surface tracer and with leaf staging
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) capture = cudaStreamCaptureStatusActive;
-    if (c->surf) {
-        // Scenes with triangles: the surface tracer.
-        const void* kernel = vpt::surface_kernel_ptr(grid_maj, dlog != nullptr, tp.grid.st_values != nullptr);
-        int ctas = vpt::persistent_grid(c, threads, kernel, smem);
-        vpt::launch_surface(tp, grid_maj, ctas, threads, smem, s);
-    } else if (c->tracker == 1 && capture == cudaStreamCaptureStatusNone) {
+    if (c->tracker == 1 && !c->surf && capture == cudaStreamCaptureStatusNone) {
         // Wavefront tracer: its passes are issued from the host until every slot retired (not
         // capturable; a stream being captured gets one of the persistent trackers below).
         const uint64_t items = tp.stream_mode == 1 ? npix * spp : npix;
@@ -645,7 +636,8 @@ static int launch_plain_impl(VptContext* c, void* stream, uint32_t spp, uint32_t
         rc3 = vpt::wf_run(c, tp, grid_maj, smem, s);
         if (rc3) return rc3;
     } else if (stage) {
-        const size_t launch_smem = vpt::plain_smem_bytes(smem, true, threads);
+        const int threads = c->threads > 0 ? c->threads : 128;
+        const size_t launch_smem = vpt::stage_smem_bytes(smem, threads);
         const int ctas = vpt::persistent_grid(c, threads, vpt::stage_kernel_ptr(dlog != nullptr), launch_smem);
         vpt::launch_stage(tp, ctas, threads, launch_smem, s);
     } else {

@@ -113,10 +113,8 @@ __device__ __forceinline__ void to_polar_yup(V3 v, float* theta, float* phi) {
 }
 // The same result without the library remainder: for a = atan2(..) in [-pi, pi] the sum lies in
 // [pi, 3 pi], where fmod is one subtraction of 2 pi, exact by Sterbenz's lemma, so both forms agree
-// bit for bit. The radiance-cache passes use this one (their render samples mostly end at an
-// environment hit and write cache queries: render pass 4.76 -> 4.53 ms per 128 spp at 256^2);
-// the plain tracer keeps the library call, because the select changes its register allocation at
-// its 72-register bound (spills; C2 35.0 -> 37.8 ms).
+// bit for bit. The tracker with work queues uses this one (radiance-cache render samples
+// mostly end at an environment hit and write cache queries: 4.76 -> 4.53 ms per 128 spp at 256^2).
 __device__ __forceinline__ void to_polar_yup_sel(V3 v, float* theta, float* phi) {
     *theta = acosf(fminf(fmaxf(v.y, -1.0f), 1.0f));
     const float a = atan2f(-v.x, v.z) + 2 * kPi;

@@ -2,7 +2,9 @@
 // paths, and work queues (rings of slot numbers) say what each needs next: a segment to track,
 // a collision (roulette, light sample, shadow segment), the end of a shadow segment (NEE
 // contribution, phase sample, next segment), or the end of a path (accumulation, next work item,
-// camera ray). A warp takes up to 32 slots of one kind at a time.
+// camera ray). A warp takes up to 32 slots of one kind at a time. Scenes with triangle meshes have
+// two more kinds: a vertex on a triangle and the end of its shadow segment. Whichever batch starts a
+// segment there, all its lanes search the closest hit (and test the light's visibility) together.
 //
 // * Events: one kind per batch, so that the long event code (environment sampling, phase function,
 //   camera ray, segment set-up) runs with nearly full warps. The segments that a batch starts are
@@ -18,7 +20,8 @@
 // queue per CTA of 128 or of 768 threads, and 4 CTAs per SM at 64 registers were all slower. ms per
 // launch, lane-per-path form against this one: 1024^2 x 16 spp sparse 512^3 23.6 -> 16.0, 2048^2 x
 // 4 spp 1024^3 17.4 -> 11.9, dense 64^3 at 256^2 x 16 spp 0.89 -> 0.74 and x 1 spp 0.53 -> 0.45,
-// reference rules 256^2 x 8 spp 4.2 -> 2.9, a radiance-cache frame 4.27 -> 2.99.
+// reference rules 256^2 x 8 spp 4.2 -> 2.9, a radiance-cache frame 4.27 -> 2.99. With meshes, 512^2 x
+// 4 spp: the room 23.9 -> 7.1, with two spheres through the BVH 30.5 -> 10.9.
 //
 // Each path draws its random numbers in its own order whichever lane works on it, so its samples
 // are those of the other forms to the bit. The reference is the plain and radiance-cache ray-
@@ -37,6 +40,8 @@ enum : uint32_t {
     RS_ESCAPE,      // primary segment left the grid
     RS_END,         // the path ended otherwise
     RS_FETCH,       // a slot without a path
+    RS_SURFACE,     // scenes with meshes: primary segment ended on a triangle
+    RS_NEE_SURF,    // shadow segment of a surface vertex over
 };
 constexpr uint32_t kStateMask = 15u;
 constexpr uint32_t kShadow = 1u << 4;      // the tracked segment is a shadow segment
@@ -47,6 +52,8 @@ constexpr uint32_t kTermDone = 1u << 8;    // its terminal record is written
 constexpr int kSetShift = 9;               // training set (2 bits)
 constexpr int kEndShift = 11;              // end code (3 bits)
 constexpr uint32_t kEndMask = 7u << kEndShift;
+constexpr uint32_t kHit = 1u << 14;        // the primary segment ends on a triangle
+constexpr uint32_t kAtSurface = 1u << 15;  // the current vertex is on a triangle
 constexpr uint32_t kItemBits = kTrain | kUnbiased | (3u << kSetShift);  // kept over the whole path
 
 // Words of a slot. The stride is odd, so that consecutive slots lie in different banks.
@@ -75,9 +82,12 @@ enum : int {
 constexpr int kNrcWords = 4;      // primary spread, root of the path spread, last density, previous vertex
 constexpr int kPixelWords = 9;    // per-pixel streams: sums (3 doubles), running mean
 constexpr int kLogWords = 2;      // primary and shadow lookups of the sample
-constexpr int queue_words(bool grid_majorant, bool log, bool nrc, bool per_pixel) {
+// Scenes with meshes: throughput g and b, the segment's triangle and its barycentrics, the shadow
+// ray's origin, the light-side cosine over the distance and the squared distance of its sample.
+constexpr int kSurfaceWords = 10;
+constexpr int queue_words(bool grid_majorant, bool log, bool nrc, bool per_pixel, bool surfaces) {
     return ((grid_majorant ? W_DDA_END : W_DDA) + (nrc ? kNrcWords : 0) + (per_pixel ? kPixelWords : 0) +
-            (log ? kLogWords : 0)) | 1;
+            (log ? kLogWords : 0) + (surfaces ? kSurfaceWords : 0)) | 1;
 }
 
 // Slots of a CTA: half as many again as lanes, so that work waits in the queues for full batches
@@ -97,23 +107,27 @@ constexpr uint32_t kEventBatch = 48;        // slots of one event kind that call
 constexpr int kRefill = 14;                 // idle lanes of a tracking warp that are filled together
 
 // Work queues of a CTA: rings of slots per kind of work.
-enum : uint32_t { Q_VERTEX = 0, Q_NEE_DONE, Q_END, Q_TRACK, kQueues };
+enum : uint32_t { Q_VERTEX = 0, Q_NEE_DONE, Q_END, Q_TRACK, Q_SURFACE, Q_NEE_SURF };
+constexpr uint32_t queue_count(bool surfaces) { return surfaces ? 6u : 4u; }
 constexpr uint32_t kEmpty = 0xffffu;
 constexpr uint32_t kSpinLimit = 1u << 20;   // polls of a ring entry before the CTA gives up
 constexpr uint32_t kIdleSleep = 400;        // ns between polls without work
 constexpr uint32_t kIdleLimit = 1u << 22;   // such polls before a warp leaves the rest to the others
 
-template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kStencil>
-__global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_kernel(const TraceParams P) {
+template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kStencil, bool kSurfaces>
+__global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm : kQueueCtasPerSm) queue_trace_kernel(const __grid_constant__ TraceParams P) {
+    constexpr uint32_t kQueues = queue_count(kSurfaces);
     constexpr bool kNrc = kMode != kModePlain;
     constexpr bool kCombo = kMode == kModeComboNrc;
     constexpr bool kMayTrain = kMode == kModeTrainNrc || kCombo;
     constexpr bool kMayPerPixel = !kNrc && kStreams == kStreamsPerPixel;
-    constexpr int kW = queue_words(kGridMajorant, kLog, kNrc, kMayPerPixel);
+    constexpr int kW = queue_words(kGridMajorant, kLog, kNrc, kMayPerPixel, kSurfaces);
     constexpr int kBase = kGridMajorant ? W_DDA_END : W_DDA;
     constexpr int W_PSPREAD = kBase, W_SSPREAD = kBase + 1, W_LDENS = kBase + 2, W_PREV = kBase + 3;
     constexpr int W_SUM = kBase, W_MEAN = kBase + 6;
     constexpr int W_REC = kBase + (kNrc ? kNrcWords : 0) + (kMayPerPixel ? kPixelWords : 0);
+    constexpr int W_TPGB = W_REC + (kLog ? kLogWords : 0), W_HIT = W_TPGB + 2, W_EYE = W_HIT + 3, W_LPCOS = W_EYE + 3;
+    constexpr uint32_t kKept = kItemBits | kPickSun | (kSurfaces ? kHit | kAtSurface : 0u);  // bits a segment's end leaves
     const bool sample_parallel = kStreams == kStreamsRuntime ? P.stream_mode == 1 : kStreams == kStreamsSampleParallel;
 
     extern __shared__ __align__(16) uint32_t s_mem[];
@@ -141,6 +155,9 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
     const V3 bmin = v3(g.bbox_min[0], g.bbox_min[1], g.bbox_min[2]);
     const V3 bmax = v3(g.bbox_max[0], g.bbox_max[1], g.bbox_max[2]);
     const float trace_len = 2 * P.world_radius;
+    // Radiance queries locate positions in the world box, the volume's box unless there are meshes.
+    const V3 wmin = kSurfaces ? v3(P.world_min[0], P.world_min[1], P.world_min[2]) : bmin;
+    const V3 wmax = kSurfaces ? v3(P.world_max[0], P.world_max[1], P.world_max[2]) : bmax;
     uint32_t n_lookups = 0, n_vertices = 0, n_samples = 0, n_cells = 0;
     unsigned int err = 0;
 
@@ -221,11 +238,52 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
         q[W_RNG] = static_cast<uint32_t>(r.state);
         q[W_RNG + 1] = static_cast<uint32_t>(r.state >> 32);
     };
+    // The three channels of a throughput are equal in a medium; meshes have coloured ones.
+    auto ld_tp = [&](const uint32_t* q) -> RGB {
+        const float r = __uint_as_float(q[W_TP]);
+        if constexpr (kSurfaces) return rgb(r, __uint_as_float(q[W_TPGB]), __uint_as_float(q[W_TPGB + 1]));
+        return rgb(r, r, r);
+    };
+    auto st_tp = [&](uint32_t* q, RGB tp) {
+        q[W_TP] = __float_as_uint(tp.r);
+        if constexpr (kSurfaces) {
+            q[W_TPGB] = __float_as_uint(tp.g);
+            q[W_TPGB + 1] = __float_as_uint(tp.b);
+        }
+    };
+    auto nee_state = [&](uint32_t st) -> uint32_t {
+        return kSurfaces && (st & kAtSurface) ? RS_NEE_SURF : RS_NEE_DONE;
+    };
     auto is_train = [&](uint32_t st) -> bool { return kMode == kModeTrainNrc || (kCombo && (st & kTrain)); };
     // Record index of an item in the pass buffers.
     auto record_of = [&](const uint32_t* q, uint32_t st) -> uint32_t {
         if (is_train(st) || !sample_parallel) return q[W_PIXEL];
         return q[W_SAMPLE] * num_pixels + q[W_PIXEL];
+    };
+
+    // The path ends at a vertex whose cache query was just written (optix_pathtracing_kernels.cu
+    // :307-330): the training suffix's terminal record, or the render path's terminal info and,
+    // when the render queries are listed, its record in the inference list.
+    auto end_with_query = [&](const uint32_t* q, uint32_t s, uint32_t rec, uint32_t path_length, RGB tp) {
+        if (is_train(s)) {
+            tr_suffix(s)[rec] = pack_suffix(q[W_PREV], 1, path_length, s & kUnbiased ? 1 : 0);
+            return;
+        }
+        TerminalInfo ti;
+        ti.tp[0] = tp.r;
+        ti.tp[1] = tp.g;
+        ti.tp[2] = tp.b;
+        ti.bits = 1u | ((path_length & 0xFFu) << 1);
+        P.nrc.infer_terminal[rec] = ti;
+        if (P.nrc.infer_index) {
+            // One atomic per converged group.
+            const uint32_t m = __activemask();
+            const int leader = __ffs(m) - 1;
+            uint32_t base = 0;
+            if (static_cast<int>(lane) == leader) base = atomicAdd(P.nrc.counters + 8, __popc(m));
+            base = __shfl_sync(m, base, leader);
+            P.nrc.infer_index[base + __popc(m & ((1u << lane) - 1u))] = rec;
+        }
     };
 
     // Segment set-up at the clip box: false when the ray misses it.
@@ -256,7 +314,8 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
     // takes each entry once it is there (the wait for an entry being written is bounded).
     auto push_states = [&](bool pred, uint32_t slot, uint32_t st) {
         const uint32_t s = st & kStateMask;
-        const uint32_t queue = s == RS_TRACK ? Q_TRACK : (s == RS_VERTEX ? Q_VERTEX : (s == RS_NEE_DONE ? Q_NEE_DONE : Q_END));
+        uint32_t queue = s == RS_TRACK ? Q_TRACK : (s == RS_VERTEX ? Q_VERTEX : (s == RS_NEE_DONE ? Q_NEE_DONE : Q_END));
+        if constexpr (kSurfaces) queue = s == RS_SURFACE ? Q_SURFACE : (s == RS_NEE_SURF ? Q_NEE_SURF : queue);
         __threadfence_block();
         uint32_t rest = __ballot_sync(0xffffffffu, pred && s != RS_DONE);
         const uint32_t done = __ballot_sync(0xffffffffu, pred && s == RS_DONE);
@@ -348,9 +407,17 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
         // Full event batches first, then tracking, then what there is.
         const uint32_t active = __ballot_sync(0xffffffffu, act);
         const volatile uint32_t* sv = s_mem;
-        const uint32_t c0 = count_of(sv[0]), c1 = count_of(sv[1]), c2 = count_of(sv[2]), c3 = count_of(sv[3]);
-        const uint32_t most = max(c0, max(c1, c2));
+        const uint32_t c0 = count_of(sv[Q_VERTEX]), c1 = count_of(sv[Q_NEE_DONE]), c2 = count_of(sv[Q_END]);
+        const uint32_t c3 = count_of(sv[Q_TRACK]);
+        uint32_t most = max(c0, max(c1, c2));
         uint32_t kind = c0 == most ? 0u : (c1 == most ? 1u : 2u);
+        if constexpr (kSurfaces) {
+            const uint32_t c4 = count_of(sv[Q_SURFACE]), c5 = count_of(sv[Q_NEE_SURF]);
+            if (max(c4, c5) > most) {
+                kind = c4 >= c5 ? Q_SURFACE : Q_NEE_SURF;
+                most = max(c4, c5);
+            }
+        }
         if (active || (most < kEventBatch && c3 > 0 && (c3 >= 32 || c3 >= most))) kind = Q_TRACK;
         if (sv[kQueues] == 0 || sv[kQueues + 1] != 0) kind = kQueues;
         kind = __shfl_sync(0xffffffffu, kind, 0);
@@ -369,19 +436,21 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
             bool segment = false;
             V3 seg_eye = v3(0, 0, 0), seg_dir = v3(0, 0, 1);
             float seg_max = 1e10f;
+            bool light = false;  // scenes with meshes: a light sample for the vertex at seg_eye
+            Pcg32 rng{0};
             st = RS_DONE;
             if (kind == Q_VERTEX) {
                 // Primary collision (optix_pathtracing_kernels.cu:176-182, 254-268, 282-332) and
                 // light sample (renderer_kernel_common.h:297-358).
                 if (slot != kEmpty) {
                     uint32_t* q = slot_ptr(slot);
-                    uint32_t s = q[W_ST] & ~(kStateMask | kShadow | kPickSun);
-                    Pcg32 rng = ld_rng(q);
+                    uint32_t s = q[W_ST] & kItemBits;
+                    rng = ld_rng(q);
                     const V3 seg_origin = ld3(q, W_ORG), dir = ld3(q, W_DIR);
                     const V3 origin = seg_origin + ldf(q, W_T) * dir;
                     st3(q, W_ORG, origin);
                     const uint32_t path_length = q[W_LEN];
-                    float tp = ldf(q, W_TP);
+                    RGB tp = ld_tp(q);
                     float primary_spread = 0.0f, sqrt_spread = 0.0f;
                     if constexpr (kNrc) {
                         primary_spread = ldf(q, W_PSPREAD);
@@ -400,7 +469,7 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                     bool rr_kill = false;
                     const int32_t rr_from = is_train(s) ? max(P.rr_start, 3) : P.rr_start;
                     if (static_cast<int32_t>(path_length) >= rr_from) {
-                        continue_prob = fminf(luminance(rgb(tp, tp, tp)) / ldf(q, W_INIT), 1.0f);
+                        continue_prob = fminf(luminance(tp) / ldf(q, W_INIT), 1.0f);
                         if (rng.uniform() >= continue_prob) rr_kill = true;
                     }
                     bool over = false;
@@ -422,33 +491,21 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                                 P.nrc_density_query && P.density_coeff > 0 ? ldf(q, W_LDENS) / P.density_coeff : 0.0f;
                             const uint32_t rec = record_of(q, s);
                             float* qdst = is_train(s) ? tr_end_query(s) : P.nrc.infer_query;
-                            write_query(qdst + kQueryFloats * static_cast<size_t>(rec), origin, -dir, rough, P.albedo, bmin,
-                                        bmax);
-                            if (is_train(s)) {
-                                tr_suffix(s)[rec] = pack_suffix(q[W_PREV], 1, path_length, s & kUnbiased ? 1 : 0);
-                            } else {
-                                TerminalInfo ti;
-                                ti.tp[0] = ti.tp[1] = ti.tp[2] = tp;
-                                ti.bits = 1u | ((path_length & 0xFFu) << 1);
-                                P.nrc.infer_terminal[rec] = ti;
-                                if (P.nrc.infer_index) {
-                                    // List the slot for the inference (one atomic per converged group).
-                                    const uint32_t m = __activemask();
-                                    const int leader = __ffs(m) - 1;
-                                    uint32_t base = 0;
-                                    if (static_cast<int>(lane) == leader) base = atomicAdd(P.nrc.counters + 8, __popc(m));
-                                    base = __shfl_sync(m, base, leader);
-                                    P.nrc.infer_index[base + __popc(m & ((1u << lane) - 1u))] = rec;
-                                }
-                            }
+                            write_query(qdst + kQueryFloats * static_cast<size_t>(rec), origin, -dir, rough, P.albedo, wmin,
+                                        wmax);
+                            end_with_query(q, s, rec, path_length, tp);
                             s |= RS_END | kTermDone | (END_CACHE << kEndShift);
                             over = true;
                         }
                     }
                     if (!over) {
-                        const float rcp = 1.0f / continue_prob;
-                        tp = tp * rcp;
-                        stf(q, W_TP, tp);
+                        tp = rdiv(tp, continue_prob);
+                        st_tp(q, tp);
+                    }
+                    if (kSurfaces && !over) {
+                        light = true;
+                        seg_eye = origin;
+                    } else if (!over) {
                         const float u_light = rng.uniform();
                         const float u0 = rng.uniform();
                         const float u1 = rng.uniform();
@@ -500,6 +557,220 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                     st_rng(q, rng);
                     st = s;
                 }
+            } else if (kSurfaces && kind == Q_SURFACE) {
+                // A triangle hit (optix_pathtracing_kernels.cu:176-239, 254-330): the surface point, its
+                // emission weighted against area-light sampling, roulette, light sample.
+                if (slot != kEmpty) {
+                    uint32_t* q = slot_ptr(slot);
+                    uint32_t s = (q[W_ST] & kItemBits) | kAtSurface;
+                    rng = ld_rng(q);
+                    const SurfPoint sp = surface_point(P.surf, q[W_HIT], ldf(q, W_HIT + 1), ldf(q, W_HIT + 2), P.env_enabled != 0);
+                    const V3 ray_origin = ld3(q, W_ORG), dir = ld3(q, W_DIR), origin = sp.pos;
+                    st3(q, W_ORG, origin);
+                    const float dir_pdf = ldf(q, W_DPDF);
+                    const uint32_t path_length = q[W_LEN];
+                    RGB tp = ld_tp(q);
+                    const V3 vout_local = to_local(sp.sf, -dir);
+                    const SurfMaterial& mt = P.surf.mats[sp.material];
+                    float primary_spread = 0.0f, sqrt_spread = 0.0f;
+                    if constexpr (kNrc) {
+                        // :200-210: path spread, |cos| against the geometric normal.
+                        primary_spread = ldf(q, W_PSPREAD);
+                        sqrt_spread = ldf(q, W_SSPREAD);
+                        const V3 dv = ray_origin - origin;
+                        const float dist2 = dv.x * dv.x + dv.y * dv.y + dv.z * dv.z;
+                        const float abs_dot = fabsf(dot(dir, sp.gn));
+                        if (path_length == 1) {
+                            primary_spread = dist2 / (4 * kPi * abs_dot);
+                            stf(q, W_PSPREAD, primary_spread);
+                        } else {
+                            sqrt_spread += sqrtf(dist2 / (dir_pdf * abs_dot));
+                            stf(q, W_SSPREAD, sqrt_spread);
+                        }
+                    }
+                    if (vout_local.z > 0 && mt.emissive) {
+                        const RGB em = rgb(mt.emittance[0], mt.emittance[1], mt.emittance[2]);
+                        float mis = 1.0f;
+                        if (path_length > 1) {
+                            const V3 dv = ray_origin - origin;
+                            const float dist2 = dot(dv, dv);
+                            const float light_pdf = sp.hyp_area_pdf * dist2 / vout_local.z;
+                            const float bsdf_pdf = dir_pdf;
+                            mis = (bsdf_pdf * bsdf_pdf) / ((bsdf_pdf * bsdf_pdf) + (light_pdf * light_pdf));
+                        }
+                        const RGB implicit = em * (mis / kPi);
+                        if (!is_train(s)) {
+                            const V3 c = ld3(q, W_CON);
+                            const RGB add = tp * implicit;
+                            st3(q, W_CON, v3(c.x + add.r, c.y + add.g, c.z + add.b));
+                        } else if (q[W_PREV] != kInvalidVertex) {
+                            // :231-237: the emission completes the previous vertex's target.
+                            const TrainVertexInfo& pv = tr_vertex(s)[q[W_PREV]];
+                            float* tg = tr_target0(s) + 3 * static_cast<size_t>(q[W_PREV]);
+                            const RGB add = rgb(pv.local_tp[0], pv.local_tp[1], pv.local_tp[2]) * implicit;
+                            tg[0] += add.r;
+                            tg[1] += add.g;
+                            tg[2] += add.b;
+                        }
+                    }
+                    float continue_prob = 1.0f;
+                    bool rr_kill = false;
+                    const int32_t rr_from = is_train(s) ? max(P.rr_start, 3) : P.rr_start;
+                    if (static_cast<int32_t>(path_length) >= rr_from) {
+                        continue_prob = fminf(luminance(tp) / ldf(q, W_INIT), 1.0f);
+                        if (rng.uniform() >= continue_prob) rr_kill = true;
+                    }
+                    bool over = false;
+                    if constexpr (!kNrc) {
+                        if (rr_kill) {
+                            s |= RS_END | (END_RR << kEndShift);
+                            over = true;
+                        }
+                    } else {
+                        // :282-330 at a surface: the query holds the shading normal and the material's
+                        // reflectances and roughness.
+                        bool ends_with_cache = rr_kill;
+                        const float spread2 = sqrt_spread * sqrt_spread;
+                        if (is_train(s)) {
+                            if (!(s & kUnbiased)) ends_with_cache |= spread2 > train_term_factor * primary_spread;
+                        } else {
+                            ends_with_cache |= spread2 > term_factor * primary_spread;
+                        }
+                        if (ends_with_cache) {
+                            const uint32_t rec = record_of(q, s);
+                            float* qdst = is_train(s) ? tr_end_query(s) : P.nrc.infer_query;
+                            write_query_surface(qdst + kQueryFloats * static_cast<size_t>(rec), origin, sp.sf.n, -dir, mt, wmin,
+                                                wmax);
+                            end_with_query(q, s, rec, path_length, tp);
+                            s |= RS_END | kTermDone | (END_CACHE << kEndShift);
+                            over = true;
+                        }
+                    }
+                    if (!over) {
+                        tp = rdiv(tp, continue_prob);
+                        st_tp(q, tp);
+                        light = true;
+                        seg_eye = origin;
+                    }
+                    st_rng(q, rng);
+                    st = s;
+                }
+            } else if (kSurfaces && kind == Q_NEE_SURF) {
+                // NEE contribution with the surface's BSDF (renderer_kernel_common.h:385-402), BSDF
+                // sample, offset origin of the next ray (optix_pathtracing_kernels.cu:340-409).
+                if (slot != kEmpty) {
+                    uint32_t* q = slot_ptr(slot);
+                    const uint32_t s_in = q[W_ST];
+                    uint32_t s = s_in & kItemBits;
+                    rng = ld_rng(q);
+                    const V3 old_dir = ld3(q, W_DIR);
+                    RGB tp = ld_tp(q);
+                    const SurfPoint sp = surface_point(P.surf, q[W_HIT], ldf(q, W_HIT + 1), ldf(q, W_HIT + 2), P.env_enabled != 0);
+                    const SurfMaterial& mt = P.surf.mats[sp.material];
+                    const Bsdf f = make_bsdf(mt);
+                    const V3 vq = to_local(sp.sf, -old_dir);
+                    RGB nee_value = rgb(0, 0, 0);
+                    const float vis = ldf(q, W_VIS);
+                    if (vis > 0.0f) {
+                        const V3 light_dir = ld3(q, W_LDIR);
+                        const float area_pdf = ldf(q, W_APDF);
+                        const float nee_lp_cos = ldf(q, W_LPCOS), nee_dist2 = ldf(q, W_LPCOS + 1);
+                        const V3 sdir = -light_dir;
+                        const V3 vin = to_local(sp.sf, -sdir);
+                        float bpdf0;
+                        const RGB fs = bsdf_eval_pdf(f, vq, vin, &bpdf0);
+                        const float sp_cos = fabsf(dot(sdir, sp.gn));
+                        RGB nee;
+                        if (s_in & kPickSun) {
+                            const RGB emittance = rgb(P.sun.irradiance[0], P.sun.irradiance[1], P.sun.irradiance[2]);
+                            nee = fs * emittance * (vis * sp_cos / area_pdf);
+                        } else {
+                            const V3 e = ld3(q, W_EMI);
+                            const RGB emittance = rgb(e.x, e.y, e.z);
+                            float bpdf = bpdf0 * nee_lp_cos / nee_dist2;
+                            if (!isfinite(bpdf)) bpdf = 0.0f;
+                            const float light_pdf = area_pdf;
+                            const float mis = (light_pdf * light_pdf) / ((bpdf * bpdf) + (light_pdf * light_pdf));
+                            const RGB le = rdiv(emittance, kPi);
+                            const float gterm = nee_lp_cos * sp_cos / nee_dist2;
+                            nee = fs * le * (vis * mis * gterm / area_pdf);
+                        }
+                        if (!is_train(s)) {
+                            const V3 c = ld3(q, W_CON);
+                            const RGB add = tp * nee;
+                            st3(q, W_CON, v3(c.x + add.r, c.y + add.g, c.z + add.b));
+                        }
+                        nee_value = nee;
+                    }
+                    uint32_t path_length = q[W_LEN];
+                    bool over = false;
+                    if (P.max_bounces > 0 && static_cast<int32_t>(path_length) >= P.max_bounces) {
+                        s |= RS_END | (END_MAX_BOUNCES << kEndShift);
+                        over = true;
+                    }
+                    if (!over) {
+                        const float u0 = rng.uniform();
+                        const float u1 = rng.uniform();
+                        V3 local;
+                        float pdf;
+                        const RGB fs = bsdf_sample(f, vq, u0, u1, &local, &pdf);
+                        if (pdf == 0.0f) {
+                            s |= RS_END | (END_PDF_ZERO << kEndShift);
+                            over = true;
+                        } else {
+                            const V3 dir = from_local(sp.sf, local);
+                            const float dot_sgn = dot(dir, sp.gn);
+                            const RGB local_tp = fs * (fabsf(dot_sgn) / pdf);
+                            tp = tp * local_tp;
+                            st_tp(q, tp);
+                            const V3 origin = offset_ray_origin(sp.pos, (dot_sgn > 0.0f ? 1.0f : -1.0f) * sp.gn);
+                            st3(q, W_ORG, origin);
+                            st3(q, W_DIR, dir);
+                            stf(q, W_DPDF, pdf);
+                            if (is_train(s)) {
+                                // :358-409 at a surface vertex: the query at the surface point (not the offset
+                                // origin), the BSDF's local throughput, the NEE target.
+                                const uint32_t prev = q[W_PREV];
+                                const uint32_t idx = atomicAdd(tr_counters(s) + tr_buf(s), 1u);
+                                if (idx < kTrainBufferSize) {
+                                    write_query_surface(tr_query0(s) + kQueryFloats * static_cast<size_t>(idx), sp.pos, sp.sf.n,
+                                                        -old_dir, mt, wmin, wmax);
+                                    TrainVertexInfo vi;
+                                    vi.local_tp[0] = local_tp.r;
+                                    vi.local_tp[1] = local_tp.g;
+                                    vi.local_tp[2] = local_tp.b;
+                                    vi.bits = (prev & kInvalidVertex) | ((path_length & 0xFFu) << 22) |
+                                              ((s & kUnbiased ? 1u : 0u) << 30);
+                                    tr_vertex(s)[idx] = vi;
+                                    float* tg = tr_target0(s) + 3 * static_cast<size_t>(idx);
+                                    tg[0] = nee_value.r;
+                                    tg[1] = nee_value.g;
+                                    tg[2] = nee_value.b;
+                                    q[W_PREV] = idx;
+                                } else {
+                                    const uint32_t rec = record_of(q, s);
+                                    write_query_surface(tr_end_query(s) + kQueryFloats * static_cast<size_t>(rec), sp.pos,
+                                                        sp.sf.n, -old_dir, mt, wmin, wmax);
+                                    tr_suffix(s)[rec] = pack_suffix(prev, 1, path_length, s & kUnbiased ? 1 : 0);
+                                    err |= VPT_DEVERR_TRAIN_FULL;
+                                    s |= RS_END | kTermDone | (END_TRAIN_FULL << kEndShift);
+                                    over = true;
+                                }
+                            }
+                            seg_eye = origin;
+                            seg_dir = dir;
+                        }
+                    }
+                    if (!over) {
+                        ++path_length;
+                        ++n_vertices;
+                        q[W_LEN] = path_length;
+                        s |= path_length > kHardVertexCap ? RS_END | (END_MAX_BOUNCES << kEndShift) : RS_ESCAPE;
+                        segment = path_length <= kHardVertexCap;
+                    }
+                    st_rng(q, rng);
+                    st = s;
+                }
             } else if (kind == Q_NEE_DONE) {
                 // NEE contribution (renderer_kernel_common.h:385-402), phase sample and next
                 // segment (optix_pathtracing_kernels.cu:341-409).
@@ -507,9 +778,9 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                     uint32_t* q = slot_ptr(slot);
                     const uint32_t s_in = q[W_ST];
                     uint32_t s = s_in & kItemBits;
-                    Pcg32 rng = ld_rng(q);
+                    rng = ld_rng(q);
                     const V3 old_dir = ld3(q, W_DIR);
-                    float tp = ldf(q, W_TP);
+                    RGB tp = ld_tp(q);
                     RGB nee_value = rgb(0, 0, 0);
                     const float vis = ldf(q, W_VIS);
                     if (vis > 0.0f) {
@@ -527,8 +798,10 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         } else {
                             const V3 e = ld3(q, W_EMI);
                             const RGB emittance = rgb(e.x, e.y, e.z);
-                            float lp_cos = dot(sdir, -light_dir);
-                            const float dist2 = 1.0f;
+                            // Scenes with meshes keep the light-side cosine over the distance and the
+                            // squared distance of an area-light sample (1 for the environment).
+                            float lp_cos = kSurfaces ? ldf(q, W_LPCOS) : dot(sdir, -light_dir);
+                            const float dist2 = kSurfaces ? ldf(q, W_LPCOS + 1) : 1.0f;
                             float bsdf_pdf = pf * lp_cos / dist2;
                             if (!isfinite(bsdf_pdf)) bsdf_pdf = 0.0f;
                             float light_pdf = area_pdf;
@@ -539,7 +812,7 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         }
                         if (!is_train(s)) {
                             const V3 c = ld3(q, W_CON);
-                            const RGB add = rgb(tp, tp, tp) * nee;
+                            const RGB add = tp * nee;
                             st3(q, W_CON, v3(c.x + add.r, c.y + add.g, c.z + add.b));
                         }
                         nee_value = nee;
@@ -564,8 +837,8 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                             RGB fs = rgb(P.albedo, P.albedo, P.albedo) * pdf;
                             dir = from_local(fr, local);
                             RGB local_tp = fs * (fabsf(1.0f) / pdf);
-                            tp = tp * local_tp.r;
-                            stf(q, W_TP, tp);
+                            tp = tp * local_tp;
+                            st_tp(q, tp);
                             st3(q, W_DIR, dir);
                             stf(q, W_DPDF, pdf);
                             if (is_train(s)) {
@@ -576,7 +849,7 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                                 const V3 origin = ld3(q, W_ORG);
                                 if (idx < kTrainBufferSize) {
                                     write_query(tr_query0(s) + kQueryFloats * static_cast<size_t>(idx), origin, -old_dir,
-                                                rough, P.albedo, bmin, bmax);
+                                                rough, P.albedo, wmin, wmax);
                                     TrainVertexInfo vi;
                                     vi.local_tp[0] = local_tp.r;
                                     vi.local_tp[1] = local_tp.g;
@@ -592,7 +865,7 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                                 } else {
                                     const uint32_t rec = record_of(q, s);
                                     write_query(tr_end_query(s) + kQueryFloats * static_cast<size_t>(rec), origin, -old_dir,
-                                                rough, P.albedo, bmin, bmax);
+                                                rough, P.albedo, wmin, wmax);
                                     tr_suffix(s)[rec] = pack_suffix(prev, 1, path_length, s & kUnbiased ? 1 : 0);
                                     err |= VPT_DEVERR_TRAIN_FULL;
                                     s |= RS_END | kTermDone | (END_TRAIN_FULL << kEndShift);
@@ -629,7 +902,7 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         if ((s & kStateMask) != RS_FETCH) {
                             const V3 c0 = ld3(q, W_CON);
                             RGB contribution = rgb(c0.x, c0.y, c0.z);
-                            const float tp = ldf(q, W_TP);
+                            const RGB tp = ld_tp(q);
                             const uint32_t path_length = q[W_LEN];
                             uint32_t end_code = (s & kEndMask) >> kEndShift;
                             if ((s & kStateMask) == RS_ESCAPE) {
@@ -639,12 +912,18 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                                     float mis = 1.0f;
                                     if (path_length > 1) {
                                         float sel = P.sun.enabled ? (1.0f - P.sun.select_prob) : 1.0f;
+                                        // :140-142: with emitting triangles the environment is picked with
+                                        // probToSampleEnvLight.
+                                        if constexpr (kSurfaces) {
+                                            if (P.surf.inst_integral > 0.0f)
+                                                sel = P.sun.enabled ? kProbEnvLight * sel : kProbEnvLight;
+                                        }
                                         float light_pdf = sel * hyp_pdf;
                                         float bsdf_pdf = ldf(q, W_DPDF);
                                         mis = (bsdf_pdf * bsdf_pdf) / ((bsdf_pdf * bsdf_pdf) + (light_pdf * light_pdf));
                                     }
                                     const RGB implicit = radiance * mis;
-                                    if (!is_train(s)) contribution = contribution + rgb(tp, tp, tp) * implicit;
+                                    if (!is_train(s)) contribution = contribution + tp * implicit;
                                     if (is_train(s)) {
                                         const uint32_t prev = q[W_PREV];
                                         if (prev != kInvalidVertex) {
@@ -670,7 +949,9 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                                 } else {
                                     if (!(s & kTermDone)) {
                                         TerminalInfo ti;
-                                        ti.tp[0] = ti.tp[1] = ti.tp[2] = tp;
+                                        ti.tp[0] = tp.r;
+                                        ti.tp[1] = tp.g;
+                                        ti.tp[2] = tp.b;
                                         ti.bits = (path_length & 0xFFu) << 1;
                                         P.nrc.infer_terminal[rec] = ti;
                                     }
@@ -740,7 +1021,6 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                             }
                         }
                         s = 0;
-                        Pcg32 rng;
                         uint32_t pixel, img_w = static_cast<uint32_t>(P.width), img_h = static_cast<uint32_t>(P.height);
                         if (kMayPerPixel && same_pixel) {
                             rng = ld_rng(q);
@@ -819,13 +1099,13 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         float az = fabsf(local.z);
                         const float dir_pdf = 1 / (az * az * az * sensor_area);
                         const float inv = 1.0f / dir_pdf;
-                        const float tp = 1.0f * inv;
+                        const RGB tp = rgb(1, 1, 1) * inv;
                         st_rng(q, rng);
                         st3(q, W_ORG, origin);
                         st3(q, W_DIR, dir);
                         stf(q, W_DPDF, dir_pdf);
-                        stf(q, W_TP, tp);
-                        stf(q, W_INIT, luminance(rgb(tp, tp, tp)));
+                        st_tp(q, tp);
+                        stf(q, W_INIT, luminance(tp));
                         st3(q, W_CON, v3(0, 0, 0));
                         q[W_LEN] = 1;
                         if constexpr (kNrc) {
@@ -842,10 +1122,128 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                     } while (false);
                 }
             }
+            if constexpr (kSurfaces) {
+                bool overflow = false;
+                if (segment) {
+                    // A primary segment ends at its closest triangle (optix_pathtracing_kernels.cu:84-96).
+                    uint32_t* q = slot_ptr(slot);
+                    const SurfHit h = bvh_closest(P.surf, seg_eye, seg_dir, 0.0f, 1e10f, &overflow);
+                    if (h.tri != ~0u) {
+                        q[W_HIT] = h.tri;
+                        stf(q, W_HIT + 1, h.b1);
+                        stf(q, W_HIT + 2, h.b2);
+                        seg_max = h.t;
+                        st = (st & ~kStateMask) | RS_SURFACE | kHit;
+                    }
+                    segment = P.volume_enabled != 0;
+                }
+                if (light) {
+                    // Light sample (renderer_kernel_common.h:297-358): the environment group (image or
+                    // sky, and the sun) against the emitting triangles with probToSampleEnvLight, the
+                    // triangles' visibility test from the light towards the vertex, then the shadow
+                    // segment through the volume.
+                    uint32_t* q = slot_ptr(slot);
+                    const V3 origin = seg_eye;
+                    float u_light = rng.uniform();
+                    const float u0 = rng.uniform();
+                    const float u1 = rng.uniform();
+                    const bool areas = P.surf.inst_integral > 0.0f;
+                    const bool env_group = P.env_enabled || P.sun.enabled;
+                    bool select_env = false, pick_sun = false;
+                    float type_prob = 1.0f;
+                    if (env_group) {
+                        if (areas) {
+                            if (u_light < kProbEnvLight) {
+                                type_prob = kProbEnvLight;
+                                u_light /= type_prob;
+                                select_env = true;
+                            } else {
+                                type_prob = 1.0f - kProbEnvLight;
+                                u_light = (u_light - kProbEnvLight) / type_prob;
+                            }
+                        } else {
+                            select_env = true;
+                        }
+                    }
+                    float nee_lp_cos = 1.0f, nee_dist2 = 1.0f, area_pdf = 1.0f;
+                    bool have_light = env_group || areas;
+                    V3 sdir = v3(0, 0, 1), light_dir = v3(0, 1, 0), shadow_eye = v3(0, 0, 0);
+                    RGB emittance = rgb(0, 0, 0);
+                    float trace_length = trace_len;
+                    if (have_light && select_env) {
+                        float light_prob = 1.0f;
+                        if (P.sun.enabled && P.env_enabled) {
+                            if (u_light < P.sun.select_prob) {
+                                pick_sun = true;
+                                light_prob = P.sun.select_prob;
+                            } else {
+                                light_prob = 1.0f - P.sun.select_prob;
+                            }
+                        } else if (P.sun.enabled) {
+                            pick_sun = true;
+                        }
+                        if (pick_sun) {
+                            light_dir = v3(P.sun.dir[0], P.sun.dir[1], P.sun.dir[2]);
+                            area_pdf = light_prob;
+                        } else {
+                            float pdf;
+                            const RGB radiance = env_sample(P.env, u0, u1, &light_dir, &pdf);
+                            emittance = kPi * radiance;
+                            area_pdf = pdf;
+                            if (area_pdf == 0.0f) have_light = false;
+                            area_pdf *= light_prob;
+                        }
+                        if (have_light) {
+                            area_pdf *= type_prob;
+                            sdir = -light_dir;
+                            nee_lp_cos = dot(sdir, -light_dir);
+                            if (nee_lp_cos <= 0.0f) have_light = false;
+                            shadow_eye = origin + trace_len * light_dir;
+                        }
+                    } else if (have_light) {
+                        const AreaSample as = sample_area_light(P.surf, u_light, u0, u1);
+                        if (as.area_pdf == 0.0f) {
+                            have_light = false;
+                        } else {
+                            area_pdf = as.area_pdf * type_prob;
+                            emittance = as.emittance;
+                            sdir = origin - as.pos;
+                            const float lp_cos = dot(sdir, as.normal);
+                            if (lp_cos <= 0.0f) {
+                                have_light = false;
+                            } else {
+                                shadow_eye = offset_ray_origin(as.pos, as.normal);
+                                sdir = origin - shadow_eye;
+                                nee_dist2 = dot(sdir, sdir);
+                                trace_length = sqrtf(nee_dist2);
+                                sdir = sdir * (1.0f / trace_length);
+                                nee_lp_cos = lp_cos / trace_length;
+                                light_dir = -sdir;
+                            }
+                        }
+                    }
+                    if (have_light && bvh_any(P.surf, shadow_eye, sdir, 0.0f, trace_length * 0.9999f, &overflow))
+                        have_light = false;
+                    st3(q, W_LDIR, light_dir);
+                    st3(q, W_EMI, v3(emittance.r, emittance.g, emittance.b));
+                    stf(q, W_APDF, area_pdf);
+                    stf(q, W_LPCOS, nee_lp_cos);
+                    stf(q, W_LPCOS + 1, nee_dist2);
+                    st3(q, W_EYE, shadow_eye);
+                    stf(q, W_VIS, have_light ? 1.0f : 0.0f);
+                    st_rng(q, rng);
+                    st |= nee_state(st) | (pick_sun ? kPickSun : 0u);
+                    segment = have_light && P.volume_enabled;
+                    seg_eye = shadow_eye;
+                    seg_dir = sdir;
+                    seg_max = trace_length;
+                }
+                if (overflow) err |= VPT_DEVERR_BVH_STACK;
+            }
             if (slot != kEmpty) {
                 uint32_t* q = slot_ptr(slot);
                 if (segment && start_segment(q, seg_eye, seg_dir, seg_max))
-                    st = (st & ~kStateMask) | RS_TRACK | (kind == Q_VERTEX ? kShadow : 0u);
+                    st = (st & ~kStateMask) | RS_TRACK | (kind == Q_VERTEX || (kSurfaces && kind == Q_SURFACE) ? kShadow : 0u);
                 q[W_ST] = st;
                 // The segments that start here are tracked by this warp at once.
                 give = (st & kStateMask) != RS_TRACK;
@@ -870,7 +1268,10 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
             eye = ld3(q, W_ORG);
             if (st & kShadow) {
                 const V3 light_dir = ld3(q, W_LDIR);
-                eye = eye + trace_len * light_dir;
+                if constexpr (kSurfaces)
+                    eye = ld3(q, W_EYE);
+                else
+                    eye = eye + trace_len * light_dir;
                 dir = -light_dir;
             }
             steps = steps0 = q[W_STEPS];
@@ -942,7 +1343,11 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         maj = P.density_coeff * maj_grid[lin];
                     }
                 }
-                if (!act) next = st & kShadow ? RS_NEE_DONE : RS_ESCAPE;
+                if constexpr (kSurfaces) {
+                    if (!act) next = st & kShadow ? nee_state(st) : (st & kHit ? RS_SURFACE : RS_ESCAPE);
+                } else {
+                    if (!act) next = st & kShadow ? RS_NEE_DONE : RS_ESCAPE;
+                }
             }
             if (lookup) {
                 const V3 xyz = world_to_index(g, eye + dir * t);
@@ -961,7 +1366,10 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                         if (rng.uniform() >= p) {
                             vis = 0.0f;
                             act = false;
-                            next = RS_NEE_DONE;
+                            if constexpr (kSurfaces)
+                                next = nee_state(st);
+                            else
+                                next = RS_NEE_DONE;
                         } else {
                             vis = rr_thr;
                         }
@@ -985,13 +1393,14 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
                 break;
         }
         // Hand over the ended segments; all of them when a full event batch waits.
-        const bool leave = max(count_of(sv[0]), max(count_of(sv[1]), count_of(sv[2]))) >= kEventBatch;
+        bool leave = max(count_of(sv[Q_VERTEX]), max(count_of(sv[Q_NEE_DONE]), count_of(sv[Q_END]))) >= kEventBatch;
+        if (kSurfaces) leave = leave || max(count_of(sv[Q_SURFACE]), count_of(sv[Q_NEE_SURF])) >= kEventBatch;
         const bool all = __shfl_sync(0xffffffffu, leave, 0);
         if (slot != kEmpty && !give && (!act || all)) {
             uint32_t* q = slot_ptr(slot);
             n_lookups += steps - steps0;
             if constexpr (kLog) q[W_REC + (st & kShadow ? 1 : 0)] += steps - steps0;
-            st = (st & (kItemBits | kPickSun)) | next;
+            st = (st & kKept) | next;
             q[W_ST] = st;
             st_rng(q, rng);
             stf(q, W_T, t);
@@ -1034,44 +1443,42 @@ __global__ void __launch_bounds__(kQueueThreads, kQueueCtasPerSm) queue_trace_ke
     }
 }
 
-template <bool kGridMajorant, bool kLog, int kMode, int kStreams>
+template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kSurfaces>
 const void* kernel_of(bool stencil) {
-    return stencil ? reinterpret_cast<const void*>(queue_trace_kernel<kGridMajorant, kLog, kMode, kStreams, true>)
-                   : reinterpret_cast<const void*>(queue_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false>);
+    return stencil ? reinterpret_cast<const void*>(queue_trace_kernel<kGridMajorant, kLog, kMode, kStreams, true, kSurfaces>)
+                   : reinterpret_cast<const void*>(queue_trace_kernel<kGridMajorant, kLog, kMode, kStreams, false, kSurfaces>);
 }
-template <bool kLog, int kMode, int kStreams>
+template <bool kLog, int kMode, int kStreams, bool kSurfaces>
 const void* kernel_of(bool grid_majorant, bool stencil) {
-    return grid_majorant ? kernel_of<true, kLog, kMode, kStreams>(stencil)
-                         : kernel_of<false, kLog, kMode, kStreams>(stencil);
+    return grid_majorant ? kernel_of<true, kLog, kMode, kStreams, kSurfaces>(stencil)
+                         : kernel_of<false, kLog, kMode, kStreams, kSurfaces>(stencil);
+}
+
+template <bool kSurfaces>
+const void* kernel_ptr(int mode, bool grid_majorant, bool logged, bool sample_parallel, bool stencil) {
+    if (mode == kModeTrainNrc) return kernel_of<false, kModeTrainNrc, kStreamsRuntime, kSurfaces>(grid_majorant, stencil);
+    if (mode == kModeComboNrc) return kernel_of<false, kModeComboNrc, kStreamsRuntime, kSurfaces>(grid_majorant, stencil);
+    if (mode == kModeRenderNrc) return kernel_of<false, kModeRenderNrc, kStreamsRuntime, kSurfaces>(grid_majorant, stencil);
+    if (logged)
+        return sample_parallel ? kernel_of<true, kModePlain, kStreamsSampleParallel, kSurfaces>(grid_majorant, stencil)
+                               : kernel_of<true, kModePlain, kStreamsPerPixel, kSurfaces>(grid_majorant, stencil);
+    return sample_parallel ? kernel_of<false, kModePlain, kStreamsSampleParallel, kSurfaces>(grid_majorant, stencil)
+                           : kernel_of<false, kModePlain, kStreamsPerPixel, kSurfaces>(grid_majorant, stencil);
 }
 
 }  // namespace
 
-const void* queue_kernel_ptr(int mode, bool grid_majorant, bool logged, bool sample_parallel, bool stencil) {
-    if (mode == kModeTrainNrc) return kernel_of<false, kModeTrainNrc, kStreamsRuntime>(grid_majorant, stencil);
-    if (mode == kModeComboNrc) return kernel_of<false, kModeComboNrc, kStreamsRuntime>(grid_majorant, stencil);
-    if (mode == kModeRenderNrc) return kernel_of<false, kModeRenderNrc, kStreamsRuntime>(grid_majorant, stencil);
-    if (logged)
-        return sample_parallel ? kernel_of<true, kModePlain, kStreamsSampleParallel>(grid_majorant, stencil)
-                               : kernel_of<true, kModePlain, kStreamsPerPixel>(grid_majorant, stencil);
-    return sample_parallel ? kernel_of<false, kModePlain, kStreamsSampleParallel>(grid_majorant, stencil)
-                           : kernel_of<false, kModePlain, kStreamsPerPixel>(grid_majorant, stencil);
-}
-
-size_t queue_smem_bytes(int mode, bool grid_majorant, bool logged, bool sample_parallel, int threads, size_t maj_bytes) {
-    const bool nrc = mode != kModePlain;
-    const size_t words = queue_words(grid_majorant, logged, nrc, !nrc && !sample_parallel);
-    return 32 + queue_slots(threads) * words * 4 + kQueues * queue_ring(threads) * 2 + maj_bytes;
-}
-
 cudaError_t launch_queues(TraceParams& p, int mode, bool grid_majorant, int threads, int ctas_per_sm, int sms,
                           cudaStream_t s) {
-    const bool logged = p.dlog != nullptr, sample_parallel = p.stream_mode == 1;
+    const bool logged = p.dlog != nullptr, sample_parallel = p.stream_mode == 1, nrc = mode != kModePlain;
+    const bool surfaces = p.surf.enabled != 0, stencil = p.grid.st_values != nullptr;
     const int cells = grid_majorant ? p.grid.mx * p.grid.my * p.grid.mz : 0;
     p.maj_in_smem = cells > 0 && cells <= kQueueMajCells;
-    const void* kernel = queue_kernel_ptr(mode, grid_majorant, logged, sample_parallel, p.grid.st_values != nullptr);
-    const size_t smem = queue_smem_bytes(mode, grid_majorant, logged, sample_parallel, threads,
-                                         p.maj_in_smem ? cells * sizeof(float) : 0);
+    const void* kernel = surfaces ? kernel_ptr<true>(mode, grid_majorant, logged, sample_parallel, stencil)
+                                  : kernel_ptr<false>(mode, grid_majorant, logged, sample_parallel, stencil);
+    const size_t words = queue_words(grid_majorant, logged, nrc, !nrc && !sample_parallel, surfaces);
+    const size_t smem = 32 + queue_slots(threads) * words * 4 + queue_count(surfaces) * queue_ring(threads) * 2 +
+                        (p.maj_in_smem ? cells * sizeof(float) : 0);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     if (ctas_per_sm <= 0 &&

@@ -83,29 +83,22 @@ constexpr int kMajSmemCells = 8192;
 void launch_stage(const TraceParams& p, int grid_ctas, int threads, size_t smem, cudaStream_t s);
 // Dynamic shared memory of such a launch: the staged majorant grid (`maj_bytes`, 0 if not
 // staged), one 2 KB leaf buffer and one mbarrier per warp.
-size_t plain_smem_bytes(size_t maj_bytes, bool leaf_stage, int threads);
+size_t stage_smem_bytes(size_t maj_bytes, int threads);
 const void* stage_kernel_ptr(bool logged);
-// Plain tracer of scenes with surfaces (either stream layout, logged or not).
-const void* surface_kernel_ptr(bool grid_majorant, bool logged, bool stencil);
-void launch_surface(const TraceParams& p, bool grid_majorant, int grid_ctas, int threads, size_t smem, cudaStream_t s);
-// The tracker with work queues (vpt_queues.cu): volume scenes, every mode, either stream layout.
+// The tracker with work queues (vpt_queues.cu): every mode, either stream layout, with or without
+// triangle meshes.
 constexpr int kQueueThreads = 256;
 constexpr int kQueueCtasPerSm = 3;
+// With meshes the BVH search needs more registers: at three CTAs (80 registers) it spills, room with
+// two spheres 12.0 ms per 4 spp at 512^2; one CTA 12.2; two (128 registers) 10.9.
+constexpr int kQueueMeshCtasPerSm = 2;
 // Majorant grids up to this many cells are staged in each CTA's shared memory (512 cells: dense
 // 64^3 launch 0.747 -> 0.739 ms, radiance-cache frame 3.04 -> 2.99 ms; 4096 cells take the L1 from
 // the gathers, sparse 512^3 16.0 -> 19.0 ms).
 constexpr int kQueueMajCells = 1024;
-const void* queue_kernel_ptr(int mode, bool grid_majorant, bool logged, bool sample_parallel, bool stencil);
-// Dynamic shared memory of a launch of `threads` threads per CTA.
-size_t queue_smem_bytes(int mode, bool grid_majorant, bool logged, bool sample_parallel, int threads, size_t maj_bytes);
 // One launch with `threads` threads per CTA on `ctas_per_sm` x `sms` CTAs (0 = as many as fit).
 cudaError_t launch_queues(TraceParams& p, int mode, bool grid_majorant, int threads, int ctas_per_sm, int sms,
                           cudaStream_t s);
-// Radiance-cache render (kModeRenderNrc), training (kModeTrainNrc) or combined (kModeComboNrc)
-// pass of a scene with triangle meshes.
-void launch_nrc_surfaces(const TraceParams& p, int mode, bool grid_majorant, int grid_ctas, int threads, size_t smem,
-                         cudaStream_t s);
-const void* nrc_surface_kernel_ptr(int mode, bool grid_majorant, bool stencil);
 // Jump table of sample-parallel streams first .. first + count - 1, computed on the device.
 void launch_sample_jump_table(ulonglong2* out, uint32_t first, uint32_t count, cudaStream_t s);
 void launch_finalize_mean(const double* sum, float* mean, uint32_t n_values, uint32_t samples, cudaStream_t s);

@@ -146,3 +146,36 @@ def test_surface_info_and_rejected_input(cuda_device):
     r.set_surfaces(None)
     assert r.surface_info()["triangles"] == 0
     r.close()
+
+
+@pytest.mark.parametrize("bvh", [False, True])
+@pytest.mark.parametrize("width,height,spp,threads,ctas", [(1, 1, 1, 0, 0), (3, 2, 5, 32, 1), (33, 17, 3, 96, 0),
+                                                          (31, 29, 9, 128, 2), (130, 97, 2, 0, 0)])
+def test_launch_shapes(cuda_device, width, height, spp, threads, ctas, bvh):
+    """Fewer paths than slots, CTAs of one warp up to the default, slots refilled many times: a path
+    is the same wherever it runs, so logs and states equal those of CTAs of two warps to the bit
+    (the tests above compare the default shape with the oracle)."""
+    import torch
+
+    scene = S.room_scene()
+    if bvh:
+        scene.add(S.sphere(0.22, 5, 16, 8), S.translation(0.05, 0.05, 0.4))
+    for base in (C_ROOM, C_ROOM_REFERENCE_MODE):
+        cfg = base.replace(width=width, height=height, surfaces=None)
+        out = []
+        for shape in ((ctas, threads), (1, 64)):
+            r = Renderer(width, height)
+            setup_scene(r, cfg, volume=orc.fbm_volume(cfg.volume))
+            r.set_surfaces(scene)
+            r.set_launch_shape(shape[0], shape[1], 0)
+            log = torch.zeros(width * height * spp * 4, dtype=torch.int32, device="cuda")
+            r.launch_plain_logged(spp, log.data_ptr())
+            r.synchronize()
+            out.append((log.cpu().numpy(), r.rng_states(), r.download_sum()[0], r.counters(), r.device_errors()))
+            r.close()
+        a, b = out
+        np.testing.assert_array_equal(a[0], b[0])
+        np.testing.assert_array_equal(a[1], b[1])
+        np.testing.assert_allclose(a[2], b[2], rtol=1e-12, atol=1e-15)   # FP64 atomics in launch order
+        assert a[3] == b[3] and a[4] == b[4] == 0
+        assert a[3]["samples"] == width * height * spp
