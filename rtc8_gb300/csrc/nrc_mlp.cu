@@ -609,6 +609,12 @@ __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const Ne
 // one group runs its epilogue or encodes its next input, the tensor cores serve another: G tiles
 // in flight per SM instead of one per CTA. A group reuses its input tile's shared memory for the
 // hidden activations (a layer's MMA has completed before its epilogue overwrites the operand).
+// What bounds it (one tile of the volume network, 10.4k cycles with four groups on an SM): the tensor
+// pipe at N = 64 (29 MMAs at 78-90 cycles each), then the encoder (1.9k). Encoder warps of their own
+// were slower (4 M volume queries 304 -> 354 us). Small batches are bound by latency: one bulk copy
+// brings the weights while the first queries load, and the tiles go to the SMs in turn (us, before
+// this / now: up to 24,000 queries volume 10.3 / 8.2, reference 8.2 / 6.2, hash grid 22.6 / 12.4;
+// 100,000 volume 18.5 / 14.4; 1 M 83.5 / 82.4; 4 M 292 / 288).
 __host__ __device__ constexpr uint32_t infer_tile_bytes(int in_dim) { return (kTile * in_dim * 2 + 1023) / 1024 * 1024; }
 
 // TA: the hidden activations stay in tensor memory (32 packed FP16 columns per group next to the
@@ -631,15 +637,16 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
     uint8_t* s_w = smem;
     uint8_t* s_t = smem + align_up(ly.blob_bytes, 1024) + g * kTileBytes;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + align_up(ly.blob_bytes, 1024) + G * kTileBytes);
-    uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_bar + G);
+    uint64_t* s_wbar = s_bar + G;                 // the weights have arrived
+    uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_wbar + 1);
 
-    for (uint32_t i = tid; i < ly.blob_bytes / 16; i += kTile * G)
-        reinterpret_cast<uint4*>(s_w)[i] = __ldg(reinterpret_cast<const uint4*>(blob) + i);
     constexpr uint32_t kCols = TA ? 128 : 64;  // TMEM columns per group
     if (warp == 0) tmem_alloc(s_slot, kCols * G);
     if (gt == 0) {
         mbar_init(s_bar + g, 1);
+        if (g == 0) mbar_init(s_wbar, 1);
         mbar_fence_init();
+        if (g == 0) bulk_load(s_w, blob, ly.blob_bytes, s_wbar);
     }
     fence_async_smem();
     tc_fence_before();
@@ -663,9 +670,12 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
         }
     };
     const uint32_t stride = gridDim.x * G;
-    load_query(in, idx, (blockIdx.x * G + g) * kTile + gt, n, q);
-    load_features((blockIdx.x * G + g) * kTile + gt);
-    for (uint32_t tile = blockIdx.x * G + g; tile < ntiles && ok; tile += stride) {
+    // Tiles go to the CTAs in turn, so that a batch of fewer tiles than groups uses every SM.
+    const uint32_t first = g * gridDim.x + blockIdx.x;
+    load_query(in, idx, first * kTile + gt, n, q);
+    load_features(first * kTile + gt);
+    ok = named_sync_and(bar_id, kTile, mbar_wait(s_wbar, 0));
+    for (uint32_t tile = first; tile < ntiles && ok; tile += stride) {
         const uint32_t row = tile * kTile + gt;
         if constexpr (FEAT)
             encode_row_features<-1>(f, q, s_t, gt);
@@ -1223,7 +1233,7 @@ __global__ void selftest_kernel(const float* __restrict__ A, const float* __rest
 constexpr bool kInferTmemActivations = true;
 constexpr uint32_t kMaxSmemOptIn = 232448;  // 227 KB per CTA
 uint32_t infer_smem(const NetLayout& l, int groups) {
-    const uint32_t s = align_up(l.blob_bytes, 1024) + groups * infer_tile_bytes(l.in_dim) + groups * 8 + 16;
+    const uint32_t s = align_up(l.blob_bytes, 1024) + groups * infer_tile_bytes(l.in_dim) + groups * 8 + 24;
     // The TA form allocates 128 TMEM columns per group, all 512 of an SM at four groups: the
     // shared-memory request keeps a second CTA off the SM so that its allocation never waits.
     return kInferTmemActivations ? std::max<uint32_t>(s, kMaxSmemOptIn / 2 + 1024) : s;
@@ -1235,9 +1245,10 @@ int infer_groups(const NetLayout& l) {
     return 1;
 }
 // Inference batches from this size on compute the hash-grid features level by level (us, fused
-// kernel against this: 16,384 queries 22.8 / 18.7, 65,536 24.7 / 20.8, 131,072 43.4 / 27.3, 2^20
-// 264 / 124, 3 M 730 / 358). Below it, three launches and 152 table loads are not worth it.
-constexpr uint32_t kFeatureMinQueries = 1u << 14;
+// kernel against this: 16,384 queries 13.2 / 16.5, 30,000 16.4 / 16.5, 40,000 20.5 / 18.4, 131,072
+// 39.5 / 26.7, 2^20 250 / 120, 4 M 966 / 476). Below it, three launches and 152 table loads are not
+// worth it.
+constexpr uint32_t kFeatureMinQueries = 1u << 15;
 template <int G>
 const void* infer_kernel_for(int enc, bool features) {
     if (enc == NRC_ENCODING_VOLUME) return reinterpret_cast<const void*>(mlp_infer_kernel<144, G, kInferTmemActivations>);
@@ -1501,7 +1512,7 @@ static int launch_infer(NrcHandle* h, cudaStream_t s, const uint32_t* grid_or_fe
                         const uint32_t* idx, const uint32_t* dev_n, uint32_t n, float* out) {
     const int G = h->infer_groups;
     const uint32_t tiles = (n + kTile - 1) / kTile;
-    const uint32_t grid = std::min<uint32_t>((tiles + G - 1) / G, static_cast<uint32_t>(h->num_sms));
+    const uint32_t grid = std::min<uint32_t>(tiles, static_cast<uint32_t>(h->num_sms));
     const uint8_t* blob = h->blob_infer;
     unsigned int* err = h->err;
     void* args[] = {&h->ly, &blob, &grid_or_features, &in, &idx, &dev_n, &n, &out, &err};

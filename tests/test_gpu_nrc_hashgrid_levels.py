@@ -26,7 +26,8 @@ def _inputs(n, seed):
     return torch.from_numpy(q).cuda()
 
 
-@pytest.mark.parametrize("n,hidden", [(16383, 2), (16384, 2), (16385, 1), (20001, 7), ((1 << 20) + 77, 2)])
+@pytest.mark.parametrize("n,hidden", [(16383, 2), (16384, 2), (16385, 1), (20001, 7), (32767, 2), (32768, 1), (32769, 7),
+                                      ((1 << 20) + 77, 2)])
 def test_levels_equal_fused(cuda_device, n, hidden):
     import torch
 
