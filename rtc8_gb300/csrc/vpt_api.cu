@@ -176,6 +176,7 @@ static int build_stencils(VptContextImpl* c) {
     int32_t* d_list = nullptr;
     int rc;
     if ((rc = dev_alloc(&c->d_st_table, cells)) || (rc = dev_alloc(&d_list, cells))) {
+        cudaGetLastError();  // no room: traced from the leaves
         dev_free(&c->d_st_table);
         return VPT_OK;
     }
