@@ -21,7 +21,11 @@
 // launch, lane-per-path form against this one: 1024^2 x 16 spp sparse 512^3 23.6 -> 16.0, 2048^2 x
 // 4 spp 1024^3 17.4 -> 11.9, dense 64^3 at 256^2 x 16 spp 0.89 -> 0.74 and x 1 spp 0.53 -> 0.45,
 // reference rules 256^2 x 8 spp 4.2 -> 2.9, a radiance-cache frame 4.27 -> 2.99. With meshes, 512^2 x
-// 4 spp: the room 23.9 -> 7.1, with two spheres through the BVH 30.5 -> 10.9.
+// 4 spp: the room 23.9 -> 6.7, with two spheres through the BVH 30.5 -> 10.2 (bound by instruction
+// fetch: a third to a half of the issue slots). Of a warp's cycles, clock64 gives on the dense / sparse
+// launch: tracking 32 / 62%, choosing, handing over and taking work 24 / 12%, collisions 8 / 10% (the
+// sparse scene's sky has 11 mip levels), the other events 10 / 5%, loading segments 8 / 6%, idle 10-18
+// / 4%.
 //
 // Each path draws its random numbers in its own order whichever lane works on it, so its samples
 // are those of the other forms to the bit. The reference is the plain and radiance-cache ray-
@@ -92,10 +96,14 @@ constexpr int queue_words(bool grid_majorant, bool log, bool nrc, bool per_pixel
 
 // Slots of a CTA: half as many again as lanes, so that work waits in the queues for full batches
 // (a quarter more: sparse 512^3 16.0 -> 16.7 ms; twice as many do not leave room for the L1).
-__host__ __device__ constexpr uint32_t queue_slots(uint32_t threads) { return threads + threads / 2; }
+// Scenes with meshes have more kinds of work and fewer CTAs: three quarters more (room / with spheres
+// through the BVH, ms per 4 spp at 512^2: a half 6.9 / 10.25, three quarters 6.7 / 10.15).
+__host__ __device__ constexpr uint32_t queue_slots(uint32_t threads, bool surfaces) {
+    return threads + (surfaces ? threads * 3 / 4 : threads / 2);
+}
 __host__ __device__ constexpr uint32_t queue_ring(uint32_t threads) {
     uint32_t n = 64;
-    while (n < queue_slots(threads)) n *= 2;
+    while (n < queue_slots(threads, true)) n *= 2;
     return n;
 }
 // Tuned together on the sparse 512^3 launch / the radiance-cache frame (ms): cells per step 1 / 2 /
@@ -114,6 +122,9 @@ constexpr uint32_t kSpinLimit = 1u << 20;   // polls of a ring entry before the 
 constexpr uint32_t kIdleSleep = 400;        // ns between polls without work
 constexpr uint32_t kIdleLimit = 1u << 22;   // such polls before a warp leaves the rest to the others
 
+// Orders the slots' words and the ring entries between the warps of a CTA.
+__device__ __forceinline__ void fence_cta() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+
 template <bool kGridMajorant, bool kLog, int kMode, int kStreams, bool kStencil, bool kSurfaces>
 __global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm : kQueueCtasPerSm) queue_trace_kernel(const __grid_constant__ TraceParams P) {
     constexpr uint32_t kQueues = queue_count(kSurfaces);
@@ -131,7 +142,7 @@ __global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm
     const bool sample_parallel = kStreams == kStreamsRuntime ? P.stream_mode == 1 : kStreams == kStreamsSampleParallel;
 
     extern __shared__ __align__(16) uint32_t s_mem[];
-    const uint32_t slots = queue_slots(blockDim.x), ring = queue_ring(blockDim.x);
+    const uint32_t slots = queue_slots(blockDim.x, kSurfaces), ring = queue_ring(blockDim.x);
     uint32_t* const s_queue = s_mem;                 // per queue: tail << 16 | head
     uint32_t* const s_live = s_mem + kQueues;        // slots with a path or an item to fetch
     uint32_t* const s_abort = s_mem + kQueues + 1;
@@ -316,25 +327,29 @@ __global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm
         const uint32_t s = st & kStateMask;
         uint32_t queue = s == RS_TRACK ? Q_TRACK : (s == RS_VERTEX ? Q_VERTEX : (s == RS_NEE_DONE ? Q_NEE_DONE : Q_END));
         if constexpr (kSurfaces) queue = s == RS_SURFACE ? Q_SURFACE : (s == RS_NEE_SURF ? Q_NEE_SURF : queue);
-        __threadfence_block();
-        uint32_t rest = __ballot_sync(0xffffffffu, pred && s != RS_DONE);
+        fence_cta();
+        // Lane k reserves the positions of queue k; lane kQueues takes ended slots off the live count.
+        const bool put = pred && s != RS_DONE;
+        uint32_t mine = 0, add = 0;
+        // (Rolled in the larger kernels, which wait for instructions: spheres 11.2 -> 10.25 ms, cache
+        // frame 2.82 -> 2.79; the plain volume kernels are 1-2% faster unrolled.)
+#pragma unroll (kSurfaces || kNrc ? 1 : 4)
+        for (uint32_t k = 0; k < kQueues; ++k) {
+            const uint32_t m = __ballot_sync(0xffffffffu, put && queue == k);
+            if (queue == k) mine = m;
+            if (lane == k) add = static_cast<uint32_t>(__popc(m)) << 16;
+        }
         const uint32_t done = __ballot_sync(0xffffffffu, pred && s == RS_DONE);
-        if (done && lane == 0) atomicSub(s_live, __popc(done));
-        while (rest) {
-            const uint32_t k = __shfl_sync(0xffffffffu, queue, __ffs(rest) - 1);
-            const bool mine = ((rest >> lane) & 1u) && queue == k;
-            const uint32_t m = __ballot_sync(0xffffffffu, mine);
-            rest &= ~m;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(s_queue + k, static_cast<uint32_t>(__popc(m)) << 16) >> 16;
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (mine) {
-                volatile uint16_t* e = s_ring + k * ring + ((base + __popc(m & ((1u << lane) - 1u))) & (ring - 1));
-                uint32_t spin = 0;
-                while (*e != kEmpty && ++spin < kSpinLimit) {}
-                if (spin >= kSpinLimit) *s_abort = 1;
-                *e = static_cast<uint16_t>(slot);
-            }
+        if (lane == kQueues) add = 0u - static_cast<uint32_t>(__popc(done));
+        uint32_t base = 0;
+        if (add) base = atomicAdd(s_mem + lane, add) >> 16;
+        base = __shfl_sync(0xffffffffu, base, queue);
+        if (put) {
+            volatile uint16_t* e = s_ring + queue * ring + ((base + __popc(mine & ((1u << lane) - 1u))) & (ring - 1));
+            uint32_t spin = 0;
+            while (*e != kEmpty && ++spin < kSpinLimit) {}
+            if (spin >= kSpinLimit) *s_abort = 1;
+            *e = static_cast<uint16_t>(slot);
         }
     };
     // Up to popc(want) slots of a queue, one to each lane in `want`; kEmpty where there is none.
@@ -364,7 +379,7 @@ __global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm
             if (slot == kEmpty) *s_abort = 1;
             *e = static_cast<uint16_t>(kEmpty);
         }
-        __threadfence_block();
+        fence_cta();
         __syncwarp();
         return slot;
     };
@@ -407,19 +422,25 @@ __global__ void __launch_bounds__(kQueueThreads, kSurfaces ? kQueueMeshCtasPerSm
         // Full event batches first, then tracking, then what there is.
         const uint32_t active = __ballot_sync(0xffffffffu, act);
         const volatile uint32_t* sv = s_mem;
-        const uint32_t c0 = count_of(sv[Q_VERTEX]), c1 = count_of(sv[Q_NEE_DONE]), c2 = count_of(sv[Q_END]);
-        const uint32_t c3 = count_of(sv[Q_TRACK]);
+        uint32_t w0, w1, w2, w3, w4, w5, w6, w7;  // the queues, then the live count and the abort flag
+        asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3)
+                     : "r"(smem_addr32(s_mem)));
+        asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w4), "=r"(w5), "=r"(w6), "=r"(w7)
+                     : "r"(smem_addr32(s_mem + 4)));
+        const uint32_t c0 = count_of(w0), c1 = count_of(w1), c2 = count_of(w2), c3 = count_of(w3);
         uint32_t most = max(c0, max(c1, c2));
         uint32_t kind = c0 == most ? 0u : (c1 == most ? 1u : 2u);
         if constexpr (kSurfaces) {
-            const uint32_t c4 = count_of(sv[Q_SURFACE]), c5 = count_of(sv[Q_NEE_SURF]);
+            const uint32_t c4 = count_of(w4), c5 = count_of(w5);
             if (max(c4, c5) > most) {
                 kind = c4 >= c5 ? Q_SURFACE : Q_NEE_SURF;
                 most = max(c4, c5);
             }
         }
         if (active || (most < kEventBatch && c3 > 0 && (c3 >= 32 || c3 >= most))) kind = Q_TRACK;
-        if (sv[kQueues] == 0 || sv[kQueues + 1] != 0) kind = kQueues;
+        if ((kSurfaces ? w6 : w4) == 0 || (kSurfaces ? w7 : w5) != 0) kind = kQueues;
         kind = __shfl_sync(0xffffffffu, kind, 0);
         if (kind == kQueues) break;
         uint32_t got = pop(kind, ~active);
@@ -1477,7 +1498,7 @@ cudaError_t launch_queues(TraceParams& p, int mode, bool grid_majorant, int thre
     const void* kernel = surfaces ? kernel_ptr<true>(mode, grid_majorant, logged, sample_parallel, stencil)
                                   : kernel_ptr<false>(mode, grid_majorant, logged, sample_parallel, stencil);
     const size_t words = queue_words(grid_majorant, logged, nrc, !nrc && !sample_parallel, surfaces);
-    const size_t smem = 32 + queue_slots(threads) * words * 4 + queue_count(surfaces) * queue_ring(threads) * 2 +
+    const size_t smem = 32 + queue_slots(threads, surfaces) * words * 4 + queue_count(surfaces) * queue_ring(threads) * 2 +
                         (p.maj_in_smem ? cells * sizeof(float) : 0);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
