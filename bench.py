@@ -687,10 +687,10 @@ def main():
     launch_s = total_ms / args.steps / 1000.0
     achieved = alg_bytes / launch_s / 1e9
     pixels = cfg.width * cfg.height
-    # The persistent tracker keeps path state in registers, so the bytes it must move are fewer:
+    # The tracker keeps path state on chip, so the bytes it must move are fewer:
     reg_bytes = 32.0 * lookups_per_launch + 88.0 * pixels
     peak, peak_kind = _peaks()
-    traffic, prof = _profile_traffic("plain_trace_kernel", args.config)
+    traffic, prof = _profile_traffic("queue_trace_kernel", args.config)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "peak_source": f"{peak_kind} hbm_gbs", "traffic_source": prof,
                 "algorithmic_bytes_per_launch": alg_bytes,

@@ -376,11 +376,11 @@ int vpt_reset_counters(VptContext* ctx);
 uint32_t vpt_get_device_errors(VptContext* ctx);
 int vpt_synchronize(VptContext* ctx, void* stream);
 
-/* Tracker of vpt_launch_plain: kind 0 = persistent megakernel (the default: one launch,
+/* Tracker of vpt_launch_plain: kind 0 = persistent tracker with work queues (the default: one launch,
  * asynchronous, capturable in a CUDA graph), 1 = wavefront: an event kernel and a persistent
  * tracking kernel alternate in passes over per-slot path state, the host issuing passes until
  * every slot retired, so the call returns once the launch's work is nearly done; a stream under
- * graph capture always gets the megakernel. slots_per_sm (paths in flight per SM, 0 = 3072),
+ * graph capture always gets the persistent one. slots_per_sm (paths in flight per SM, 0 = 3072),
  * pass_steps (lookups a segment may take per pass, 0 = 64) and track_ctas_per_sm (0 = as many
  * as fit) tune the wavefront. Both trackers draw each path's random numbers in the same order. */
 int vpt_set_tracker(VptContext* ctx, int32_t kind, int32_t slots_per_sm, int32_t pass_steps,

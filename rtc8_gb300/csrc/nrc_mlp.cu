@@ -5,9 +5,10 @@
 // first layer's operand tile, trained by a scatter-add of the first layer's input gradient, and
 // updated by the same Adam / EMA kernel as the weights.
 //
-// One CTA of 128 threads works on 128-row tiles (one thread per row): the encoded input tile
-// and every hidden activation tile are FP16 in shared memory (core-matrix layout, nrc_tc.cuh),
-// the weights are copied once per CTA into shared memory in the same layout, and each layer is
+// The kernels work on 128-row tiles (inference: one thread per row and up to four tiles per CTA;
+// training: two threads per row): the encoded input tile is FP16 in shared memory (core-matrix
+// layout, nrc_tc.cuh), the hidden activations there (training) or in tensor memory (inference), the
+// weights are copied once per CTA into shared memory in the same layout, and each layer is
 // one chain of tcgen05.mma (M = 128, N = 64 or 16, K = 16 per instruction) into an FP32 TMEM
 // accumulator, read back with tcgen05.ld for the ReLU / FP16 epilogue. Training keeps all
 // activations of a tile on chip; the backward pass reads activations and weights transposed

@@ -207,7 +207,6 @@ int launch_pass(VptContext* c, cudaStream_t s, int mode, uint32_t buf, uint32_t 
         if ((rc = vpt::upload_sample_jumps(c, spp, s))) return rc;
         tp.sample_jumps = c->d_jumps;
     }
-    tp.park_threshold = c->park_threshold;
     tp.nrc = *c->nrc;
     if (index_queries) {
         NRCP_CUDA(cudaMemsetAsync(c->nrc->counters + 8, 0, sizeof(uint32_t), s));

@@ -47,7 +47,7 @@ struct TraceParams {
     uint32_t stream_base;     // sample-parallel mode: index of the first sample of this launch
     const ulonglong2* sample_jumps;  // sample-parallel mode: LCG jump (A, C) of sample stream_base + i
     int32_t maj_in_smem;      // majorant grid staged in dynamic shared memory
-    int32_t park_threshold;   // parked lanes that trigger a warp's event phase (0 = default)
+    int32_t park_threshold;   // leaf staging: parked lanes that trigger a warp's event phase (0 = default)
     int32_t leaf_stage_min;   // > 0: per-warp leaf staging when this many lanes look up in one leaf
 
     uint64_t* rng;            // per pixel
@@ -58,7 +58,7 @@ struct TraceParams {
     unsigned long long* counters;  // lookups, vertices, samples
     unsigned int* error_flags;
 
-    // Surface scenes only (plain_trace_kernel<..., kSurfaces = true>).
+    // Surface scenes only (queue_trace_kernel<..., kSurfaces = true>).
     Surfaces surf;
     int32_t volume_enabled;   // 0: surfaces without a density grid (no tracking, no draws)
 
