@@ -1498,9 +1498,14 @@ cudaError_t launch_queues(TraceParams& p, int mode, bool grid_majorant, int thre
     const void* kernel = surfaces ? kernel_ptr<true>(mode, grid_majorant, logged, sample_parallel, stencil)
                                   : kernel_ptr<false>(mode, grid_majorant, logged, sample_parallel, stencil);
     const size_t words = queue_words(grid_majorant, logged, nrc, !nrc && !sample_parallel, surfaces);
-    const size_t smem = 32 + queue_slots(threads, surfaces) * words * 4 + queue_count(surfaces) * queue_ring(threads) * 2 +
-                        (p.maj_in_smem ? cells * sizeof(float) : 0);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    auto bytes = [&](int n, int maj_cells) -> size_t {
+        return 32 + queue_slots(n, surfaces) * words * 4 + queue_count(surfaces) * queue_ring(n) * 2 + maj_cells * sizeof(float);
+    };
+    const size_t smem = bytes(threads, p.maj_in_smem ? cells : 0);
+    // The limit is the kernel's largest launch, not this one's: threads with contexts of different
+    // shapes may launch the same kernel at once.
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(bytes(kQueueThreads, kQueueMajCells)));
     if (e != cudaSuccess) return e;
     if (ctas_per_sm <= 0 &&
         (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas_per_sm, kernel, threads, smem) != cudaSuccess ||

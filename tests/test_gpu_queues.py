@@ -42,3 +42,39 @@ def test_queues_equal_wavefront(cuda_device, width, height, spp, threads, ctas, 
         np.testing.assert_array_equal(x, y)
     np.testing.assert_allclose(a[3], b[3], rtol=1e-12, atol=1e-15)   # FP64 atomics in launch order
     assert a[4] == b[4] and a[5] == b[5] == 0
+
+
+def test_threads_with_different_launch_shapes(cuda_device):
+    """Contexts of different launch shapes and majorant grids on one kernel from several threads at once:
+    every launch succeeds and gives the single-threaded image."""
+    import threading
+
+    cfgs = [small_config_mode(size=24, n=24), small_config_mode(size=24, n=40)]
+    jobs = [(cfgs[0], 0), (cfgs[1], 32), (cfgs[0], 96), (cfgs[1], 128)]
+    want = [_render(c, volume_for(c), 2, 0, t)[2] for c, t in jobs]
+    failed = []
+
+    def work(k):
+        try:
+            c, t = jobs[k]
+            r = Renderer(c.width, c.height)
+            setup_scene(r, c, volume=volume_for(c))
+            r.set_environment_rgb(constant_environment(c.env_constant if c.env_constant is not None else 0.5))
+            r.set_launch_shape(0, t, 0)
+            for _ in range(60):
+                r.launch_plain(2)
+            r.reset_accumulation()
+            r.synchronize()
+            assert r.device_errors() == 0
+            r.close()
+        except Exception as e:  # the thread's failure is reported by the test
+            failed.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for (c, t), w in zip(jobs, want):
+        np.testing.assert_array_equal(_render(c, volume_for(c), 2, 0, t)[2], w)
