@@ -1451,25 +1451,29 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     }
     const bool vol = cfg->encoding == NRC_ENCODING_VOLUME;
     h->infer_groups = infer_groups(h->ly);
-    if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, false), infer_smem(h->ly, h->infer_groups))) ||
+    if (train_smem(h->ly) > kMaxSmemOptIn || infer_smem(h->ly, h->infer_groups) > kMaxSmemOptIn) {
+        nrc_destroy(h);
+        return fail(NRC_ERR_INVALID_ARGUMENT, "nrc_create: the network does not fit in shared memory");
+    }
+    // The limits are the hardware's, not this network's: caches of other depths share the kernels.
+    if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, false), kMaxSmemOptIn)) ||
         (rc = set_kernel_smem(vol ? reinterpret_cast<const void*>(mlp_train_kernel<144, false>)
                                   : reinterpret_cast<const void*>(mlp_train_kernel<64, false>),
-                              train_smem(h->ly)))) {
+                              kMaxSmemOptIn))) {
         nrc_destroy(h);
         return rc;
     }
     if (cfg->encoding == NRC_ENCODING_HASHGRID) {
-        if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, true),
-                                  infer_smem(h->ly, h->infer_groups))) ||
+        if ((rc = set_kernel_smem(infer_kernel_ptr(cfg->encoding, h->infer_groups, true), kMaxSmemOptIn)) ||
             (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel<false>), kEncodeSmem)) ||
             (rc = set_kernel_smem(reinterpret_cast<const void*>(grid_encode_kernel<true>), kEncodeSmem)) ||
-            (rc = set_kernel_smem(reinterpret_cast<const void*>(mlp_train_kernel<64, true>), train_smem(h->ly)))) {
+            (rc = set_kernel_smem(reinterpret_cast<const void*>(mlp_train_kernel<64, true>), kMaxSmemOptIn))) {
             nrc_destroy(h);
             return rc;
         }
-        if ((rc = alloc(&h->train_features, static_cast<size_t>(kGridLevels) * kTrainLevelsMax))) {
-            nrc_destroy(h);
-            return rc;
+        if (alloc(&h->train_features, static_cast<size_t>(kGridLevels) * kTrainLevelsMax)) {
+            cudaGetLastError();  // no room: the training kernel gathers the features itself
+            h->train_features = nullptr;
         }
         h->pool = workspace_pool(dev);
     }
@@ -1605,7 +1609,7 @@ int nrc_train(NrcHandle* h, void* stream, const float* in, const float* target, 
     };
     const uint8_t* blob = h->blob_train;
     const uint32_t* gw = h->grid_words(true);
-    if (c.encoding == NRC_ENCODING_HASHGRID && n >= kTrainLevelsMin && n <= kTrainLevelsMax) {
+    if (h->train_features && n >= kTrainLevelsMin && n <= kTrainLevelsMax) {
         uint32_t* features = h->train_features;
         const uint32_t stride = tiles * kTile;
         NRC_CUDA(cudaLaunchKernelEx(shape(std::max(h->num_sms, kGridLevels), kEncodeThreads, kEncodeSmem),

@@ -41,3 +41,36 @@ def test_batch_shapes(cuda_device, encoding, hidden):
     torch.cuda.synchronize()
     assert cache.device_errors() == 0
     cache.finalize()
+
+
+@pytest.mark.parametrize("encoding,deep", [(nrc.NRC_ENCODING_VOLUME, 5), (nrc.NRC_ENCODING_REFERENCE, 7),
+                                           (nrc.NRC_ENCODING_HASHGRID, 7)])
+def test_caches_of_different_depths(cuda_device, encoding, deep):
+    """A deep network's cache still infers and trains after a shallow one was created (they share the
+    kernels), and gives the same outputs as before."""
+    import torch
+
+    def cache(hidden):
+        cfg = nrc.default_config(encoding)
+        cfg.num_hidden_layers = hidden
+        c = nrc.NeuralRadianceCache()
+        c.initialize(config=cfg)
+        return c
+
+    n = 3000
+    q = torch.from_numpy(_queries(n, 3, volume=encoding == nrc.NRC_ENCODING_VOLUME)).cuda()
+    a, b, t = torch.zeros((n, 3), device="cuda"), torch.ones((n, 3), device="cuda"), torch.full((n, 3), 0.5, device="cuda")
+    first = cache(deep)
+    first.infer(0, q, n, a)
+    second = cache(1)
+    second.infer(0, q, n, b)
+    first.infer(0, q, n, b)
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
+    before = first.params().copy()
+    first.train(0, q, t, n)
+    second.train(0, q, t, n)
+    assert np.isfinite(first.params()).all() and (first.params() != before).any()
+    assert first.device_errors() == 0 and second.device_errors() == 0
+    first.finalize()
+    second.finalize()
