@@ -699,10 +699,12 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
                 mma_commit(s_bar + g);
             }
 
-            ok = named_sync_and(bar_id, kTile, mbar_wait(s_bar + g, phase));  // group-uniform decision
+            // Each thread waits for the product itself; the group decides whether to go on at the
+            // barrier after the epilogue (one barrier per layer).
+            ok = mbar_wait(s_bar + g, phase);
             phase ^= 1;
+            __syncwarp();
             tc_fence_after();
-            if (!ok) break;
             if (j < ly.L - 1 && TA) {
                 // ReLU + FP16 pack of the accumulator straight back into tensor memory.
 #pragma unroll
@@ -721,7 +723,7 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
                 }
                 tmem_wait_st();
                 tc_fence_before();
-                named_sync(bar_id, kTile);
+                ok = named_sync_and(bar_id, kTile, ok);
             } else if (j < ly.L - 1) {
 #pragma unroll
                 for (int c = 0; c < kWidth / 32; ++c) {  // two TMEM loads in flight per wait
@@ -734,18 +736,18 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
                 }
                 tc_fence_before();
                 fence_async_smem();
-                named_sync(bar_id, kTile);
+                ok = named_sync_and(bar_id, kTile, ok);
             } else {
                 float v[16];
                 tmem_ld16(tmem + lane_base, v);
                 tmem_wait_ld();
-                if (row < n) {
+                if (row < n && ok) {
                     float* o = out + static_cast<size_t>(record_of(idx, row)) * 3;
 #pragma unroll
                     for (int c = 0; c < 3; ++c) o[c] = ly.out_act == NRC_OUTPUT_EXP ? __expf(v[c]) : v[c];
                 }
                 tc_fence_before();
-                named_sync(bar_id, kTile);
+                ok = named_sync_and(bar_id, kTile, ok);
             }
         }
     }
