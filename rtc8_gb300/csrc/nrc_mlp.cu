@@ -615,7 +615,8 @@ __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const Ne
 // were slower (4 M volume queries 304 -> 354 us). Small batches are bound by latency: one bulk copy
 // brings the weights while the first queries load, and the tiles go to the SMs in turn (us, before
 // this / now: up to 24,000 queries volume 10.3 / 8.2, reference 8.2 / 6.2, hash grid 22.6 / 12.4;
-// 100,000 volume 18.5 / 14.4; 1 M 83.5 / 82.4; 4 M 292 / 288).
+// 100,000 volume 18.5 / 14.4; 1 M 83.5 / 82.4; 4 M 292 / 288). Each thread waits for a product itself
+// and the group meets once per layer, after the epilogue (4 M: volume 288 / 276, reference 156 / 152).
 __host__ __device__ constexpr uint32_t infer_tile_bytes(int in_dim) { return (kTile * in_dim * 2 + 1023) / 1024 * 1024; }
 
 // TA: the hidden activations stay in tensor memory (32 packed FP16 columns per group next to the
@@ -1254,7 +1255,7 @@ int infer_groups(const NetLayout& l) {
 }
 // Inference batches from this size on compute the hash-grid features level by level (us, fused
 // kernel against this: 16,384 queries 13.2 / 16.5, 30,000 16.4 / 16.5, 40,000 20.5 / 18.4, 131,072
-// 39.5 / 26.7, 2^20 250 / 120, 4 M 966 / 476). Below it, three launches and 152 table loads are not
+// 39.5 / 26.7, 2^20 250 / 114, 4 M 966 / 468). Below it, three launches and 152 table loads are not
 // worth it.
 constexpr uint32_t kFeatureMinQueries = 1u << 15;
 template <int G>
