@@ -166,12 +166,24 @@ int vpt_reset_accumulation(VptContext* c) {
 }
 
 // ------------------------------------------------------------------------------ volume
+// Gives the stencil copy back; launches then read the leaves.
+static void drop_stencils(VptContextImpl* c) {
+    dev_free(&c->d_st_table);
+    dev_free(&c->d_st_values);
+}
+
+// The volume's arrays and sizes are about to change: there is no volume until the new one is whole.
+static void begin_volume(VptContextImpl* c) {
+    drop_stencils(c);
+    c->has_volume = false;
+    c->update_world_box();
+}
+
 // Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
 // for one 32-byte load per lookup. Kept only where it takes at most half of the free device
 // memory; a larger grid is traced from its leaves.
 static int build_stencils(VptContextImpl* c) {
-    dev_free(&c->d_st_table);
-    dev_free(&c->d_st_values);
+    drop_stencils(c);
     const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
     int32_t* d_list = nullptr;
     int rc;
@@ -201,6 +213,7 @@ static int build_stencils(VptContextImpl* c) {
 
 static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, int ny, int nz, float voxel_size,
                                  const float origin[3]) {
+    begin_volume(c);
     c->nx = nx;
     c->ny = ny;
     c->nz = nz;
@@ -735,7 +748,7 @@ int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
                        const VptNanoVdbInfo& info) {
     const int64_t cells = static_cast<int64_t>(lx) * ly * lz;
     dev_free(&c->d_dense);
-    c->has_volume = false;
+    begin_volume(c);
     int32_t* d_origins = nullptr;
     int rc;
     if ((rc = dev_alloc(&c->d_cell_maj, cells)) || (rc = dev_alloc(&c->d_leaf_table, cells)) ||

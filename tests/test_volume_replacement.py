@@ -1,0 +1,41 @@
+"""Replacing a context's volume, on a stand-in for the CUDA runtime (no GPU)."""
+import pytest
+
+from . import _fake_cuda
+
+SETTERS = {
+    "dense": "lambda r, n: r.set_volume_dense(np.ones((n, n, n), np.float32), 1 / n, [-0.5] * 3)",
+    "fbm": "lambda r, n: r.generate_fbm_volume(VolumeSpec(n=n, seed=1, octaves=2), 1 / n, [-0.5] * 3)",
+    "union": "lambda r, n: r.generate_fbm_volume(VolumeSpec(n=n, seed=1, octaves=2, union_seed=2), 1 / n, [-0.5] * 3)",
+}
+
+
+@pytest.mark.parametrize("kind", list(SETTERS))
+def test_failed_replacement_leaves_the_old_volume_or_none(tmp_path, kind):
+    """Memory runs out at any allocation of a replacement: until the old volume's arrays are touched,
+    launches go on with it; from then on they are refused until a volume is set, and never see the
+    new sizes over the old arrays."""
+    out = _fake_cuda.run(f"set_volume = {SETTERS[kind]}\nclouds = {2 if kind == 'union' else 1}\n" + """
+for nth in range(1, 12):
+    r = Renderer(8, 8)
+    r.set_frame(frame_params(C1))
+    set_volume(r, 32)
+    r.launch_plain(1)
+    fake.fake_fail(MALLOC, nth)
+    why = failed(lambda: set_volume(r, 80))
+    fake.fake_fail(MALLOC, 0)
+    launches = fake.fake_calls(LAUNCH)
+    refused = failed(lambda: r.launch_plain(1))
+    if why is None:  # only the copy for faster lookups is missing
+        assert nth > clouds + 4 and refused is None and r.volume_info()["total_leaves"] == 1000
+    elif nth <= clouds:
+        assert refused is None and r.volume_info()["total_leaves"] == 64, (nth, refused)
+    else:
+        assert nth <= clouds + 4 and refused and "missing" in refused and fake.fake_calls(LAUNCH) == launches, (nth, refused)
+        assert failed(r.volume_info)
+    set_volume(r, 80)
+    r.launch_plain(1)
+    r.close()
+print("ok")
+""", tmp_path)
+    assert out.split() == ["ok"]
