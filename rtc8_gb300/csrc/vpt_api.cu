@@ -166,7 +166,8 @@ int vpt_reset_accumulation(VptContext* c) {
 }
 
 // ------------------------------------------------------------------------------ volume
-// Gives the stencil copy back; launches then read the leaves.
+// Gives the stencil copy back; launches then read the leaves. Done before a new volume's arrays are
+// allocated, so that a replacement fits wherever the volumes themselves do.
 static void drop_stencils(VptContextImpl* c) {
     dev_free(&c->d_st_table);
     dev_free(&c->d_st_values);
@@ -263,6 +264,7 @@ int vpt_set_volume_dense(VptContext* c, const float* host, int32_t nx, int32_t n
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_volume_dense: bad arguments");
     int64_t total = static_cast<int64_t>(nx) * ny * nz;
     int rc;
+    drop_stencils(c);
     if ((rc = dev_alloc(&c->d_dense, total))) return rc;
     VPT_CUDA(cudaMemcpy(c->d_dense, host, total * sizeof(float), cudaMemcpyHostToDevice));
     return build_grid_from_dense(c, c->d_dense, nx, ny, nz, voxel_size, origin);
@@ -274,6 +276,7 @@ int vpt_set_volume_dense_device(VptContext* c, const float* dev, int32_t nx, int
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_volume_dense_device: bad arguments");
     int64_t total = static_cast<int64_t>(nx) * ny * nz;
     int rc;
+    drop_stencils(c);
     if ((rc = dev_alloc(&c->d_dense, total))) return rc;
     VPT_CUDA(cudaMemcpy(c->d_dense, dev, total * sizeof(float), cudaMemcpyDeviceToDevice));
     return build_grid_from_dense(c, c->d_dense, nx, ny, nz, voxel_size, origin);
@@ -286,6 +289,7 @@ int vpt_generate_fbm_volume(VptContext* c, int32_t n, uint32_t seed, int32_t oct
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_generate_fbm_volume: bad arguments");
     int64_t total = static_cast<int64_t>(n) * n * n;
     int rc;
+    drop_stencils(c);
     if ((rc = dev_alloc(&c->d_dense, total))) return rc;
     vpt::generate_fbm(c->d_dense, n, seed, octaves, lacunarity, gain, base_frequency, threshold, c->d_scratch_u32, 0);
     VPT_CUDA(cudaGetLastError());
@@ -300,6 +304,7 @@ int vpt_generate_fbm_union(VptContext* c, int32_t n, uint32_t seed_a, uint32_t s
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_generate_fbm_union: bad arguments");
     int64_t total = static_cast<int64_t>(n) * n * n;
     int rc;
+    drop_stencils(c);
     if ((rc = dev_alloc(&c->d_dense, total))) return rc;
     float* second = nullptr;
     if ((rc = dev_alloc(&second, total))) return rc;

@@ -39,3 +39,25 @@ for nth in range(1, 12):
 print("ok")
 """, tmp_path)
     assert out.split() == ["ok"]
+
+
+@pytest.mark.parametrize("kind", list(SETTERS))
+def test_replacement_fits_without_room_for_the_copy(tmp_path, kind):
+    """A replacement of the same size needs the volume's arrays and the builder's scratch only: the copy
+    of the grid that speeds lookups up gives way to them."""
+    out = _fake_cuda.run(f"set_volume = {SETTERS[kind]}\nunion = {kind == 'union'}\n" + """
+r = Renderer(8, 8)
+empty = fake.fake_bytes()
+cells, voxels = 8 ** 3, 4 * 64 ** 3
+arrays = voxels + 2 * 4 * cells + 4 * 512          # dense voxels, two tables, one leaf
+set_volume(r, 64)
+assert fake.fake_bytes() > empty + arrays          # there is a copy
+fake.fake_limit(empty + arrays + max(4 * cells, voxels if union else 0))
+set_volume(r, 64)
+fake.fake_limit(1 << 40)
+r.set_frame(frame_params(C1))
+r.launch_plain(1)
+r.close()
+print("ok", fake.fake_bytes())
+""", tmp_path)
+    assert out.split() == ["ok", "0"]
