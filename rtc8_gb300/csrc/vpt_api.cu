@@ -48,6 +48,30 @@ void dev_free(T** p) {
     *p = nullptr;
 }
 
+// Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
+// for one 32-byte load per lookup. Taken only where it needs at most half of the free device memory;
+// a larger grid is traced from its leaves. A replacement of like size builds its copy in the old
+// one's memory (us per call, without a copy / with allocations of its own / so: 64^3 102 / 304 / 128,
+// 128^3 426 / 636 / 462, 200^3 649 / 1003 / 755; the rest is its two kernels); that
+// memory gives way where the new volume's arrays have no room beside it.
+void drop_stencils(vpt::VptContextImpl* c) {
+    dev_free(&c->d_st_table);
+    dev_free(&c->d_st_values);
+    c->st_table_cap = c->st_values_cap = 0;
+}
+
+// Memory for one of a volume's arrays.
+template <typename T>
+int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
+    int rc = dev_alloc(p, count);
+    if (rc && c->d_st_table) {
+        cudaGetLastError();
+        drop_stencils(c);
+        rc = dev_alloc(p, count);
+    }
+    return rc;
+}
+
 }  // namespace
 
 namespace vpt {
@@ -166,54 +190,54 @@ int vpt_reset_accumulation(VptContext* c) {
 }
 
 // ------------------------------------------------------------------------------ volume
-// Gives the stencil copy back; launches then read the leaves. Done before a new volume's arrays are
-// allocated, so that a replacement fits wherever the volumes themselves do.
-static void drop_stencils(VptContextImpl* c) {
-    dev_free(&c->d_st_table);
-    dev_free(&c->d_st_values);
-}
-
-// The volume's arrays and sizes are about to change: there is no volume until the new one is whole.
+// The volume's arrays and sizes are about to change: there is no volume until the new one is whole,
+// and launches on any stream have read the old one.
 static void begin_volume(VptContextImpl* c) {
-    drop_stencils(c);
+    cudaDeviceSynchronize();
     c->has_volume = false;
     c->update_world_box();
 }
 
-// Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
-// for one 32-byte load per lookup. Kept only where it takes at most half of the free device
-// memory; a larger grid is traced from its leaves.
-static int build_stencils(VptContextImpl* c) {
-    drop_stencils(c);
+// The first half, once the leaves and their table are in place: the cells' slots (and behind them, in
+// the same array, the slots' cells), their count in d_scratch_u32[1]. False where there is no room.
+static bool begin_stencils(VptContextImpl* c) {
     const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
-    int32_t* d_list = nullptr;
-    int rc;
-    if ((rc = dev_alloc(&c->d_st_table, cells)) || (rc = dev_alloc(&d_list, cells))) {
-        cudaGetLastError();  // no room: traced from the leaves
-        dev_free(&c->d_st_table);
-        return VPT_OK;
+    if (c->st_table_cap < 2 * cells || c->st_table_cap > 4 * cells) {
+        c->st_table_cap = 0;
+        if (dev_alloc(&c->d_st_table, 2 * cells)) {
+            cudaGetLastError();  // traced from the leaves
+            drop_stencils(c);
+            return false;
+        }
+        c->st_table_cap = 2 * cells;
     }
-    vpt::stencil_table(c->d_leaf_table, c->d_leaf_values, c->lx, c->ly, c->lz, c->d_st_table, d_list, c->d_scratch_u32, 0);
-    unsigned int slots = 0;
-    VPT_CUDA(cudaMemcpy(&slots, c->d_scratch_u32, sizeof(slots), cudaMemcpyDeviceToHost));
-    size_t free_bytes = 0, total_bytes = 0;
-    VPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-    const size_t values = static_cast<size_t>(std::max(slots, 1u)) * 4096;
-    if (values * sizeof(float) <= free_bytes / 2 &&
-        cudaMalloc(reinterpret_cast<void**>(&c->d_st_values), values * sizeof(float)) == cudaSuccess) {
-        vpt::stencil_fill(c->d_leaf_table, c->d_leaf_values, c->lx, c->ly, c->lz, d_list, slots, c->d_st_values, 0);
-    } else {
-        cudaGetLastError();
-        c->d_st_values = nullptr;
-        dev_free(&c->d_st_table);
+    vpt::stencil_table(c->d_leaf_table, c->d_leaf_values, c->lx, c->ly, c->lz, c->d_st_table, c->d_st_table + cells,
+                       c->d_scratch_u32 + 1, 0);
+    return true;
+}
+
+// The second half: the stencils of `slots` cells.
+static int finish_stencils(VptContextImpl* c, unsigned int slots) {
+    const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
+    const int64_t values = static_cast<int64_t>(std::max(slots, 1u)) * 4096;
+    if (c->st_values_cap < values || c->st_values_cap > 2 * values) {
+        c->st_values_cap = 0;
+        dev_free(&c->d_st_values);
+        size_t free_bytes = 0, total_bytes = 0;
+        VPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (values * sizeof(float) > free_bytes / 2 || dev_alloc(&c->d_st_values, values)) {
+            cudaGetLastError();
+            drop_stencils(c);
+            return VPT_OK;
+        }
+        c->st_values_cap = values;
     }
-    dev_free(&d_list);
+    vpt::stencil_fill(c->d_leaf_table, c->d_leaf_values, c->lx, c->ly, c->lz, c->d_st_table + cells, slots, c->d_st_values, 0);
     VPT_CUDA(cudaGetLastError());
     return VPT_OK;
 }
 
-static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, int ny, int nz, float voxel_size,
-                                 const float origin[3]) {
+static int build_grid(VptContext* c, const float* d_dense, int nx, int ny, int nz, float voxel_size, const float origin[3]) {
     begin_volume(c);
     c->nx = nx;
     c->ny = ny;
@@ -224,8 +248,8 @@ static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, in
     int64_t cells = static_cast<int64_t>(c->lx) * c->ly * c->lz;
     int32_t* d_active = nullptr;
     int rc;
-    if ((rc = dev_alloc(&d_active, cells)) || (rc = dev_alloc(&c->d_cell_maj, cells)) ||
-        (rc = dev_alloc(&c->d_leaf_table, cells)))
+    if ((rc = volume_alloc(c, &d_active, cells)) || (rc = volume_alloc(c, &c->d_cell_maj, cells)) ||
+        (rc = volume_alloc(c, &c->d_leaf_table, cells)))
         return rc;
     vpt::leaf_stats(d_dense, nx, ny, nz, c->lx, c->ly, c->lz, d_active, c->d_cell_maj, 0);
     vpt::global_max(d_dense, nx, ny, nz, c->d_scratch_u32, 0);
@@ -237,11 +261,12 @@ static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, in
     c->active_leaves = slots;
     c->total_leaves = cells;
     VPT_CUDA(cudaMemcpy(c->d_leaf_table, table.data(), cells * sizeof(int32_t), cudaMemcpyHostToDevice));
-    if ((rc = dev_alloc(&c->d_leaf_values, std::max<int64_t>(slots, 1) * 512))) return rc;
+    if ((rc = volume_alloc(c, &c->d_leaf_values, std::max<int64_t>(slots, 1) * 512))) return rc;
     vpt::pack_leaves(d_dense, nx, ny, nz, c->lx, c->ly, c->lz, c->d_leaf_table, c->d_leaf_values, 0);
-    unsigned int gmax_bits = 0;
-    VPT_CUDA(cudaMemcpy(&gmax_bits, c->d_scratch_u32, sizeof(unsigned int), cudaMemcpyDeviceToHost));
-    std::memcpy(&c->global_majorant, &gmax_bits, sizeof(float));
+    const bool stencils = begin_stencils(c);
+    unsigned int bits[2] = {0, 0};  // global majorant, slots of the stencil copy
+    VPT_CUDA(cudaMemcpy(bits, c->d_scratch_u32, sizeof(bits), cudaMemcpyDeviceToHost));
+    std::memcpy(&c->global_majorant, bits, sizeof(float));
     c->voxel_size = voxel_size;
     c->inv_voxel_size = static_cast<float>(1.0 / static_cast<double>(voxel_size));
     for (int a = 0; a < 3; ++a) c->origin[a] = origin[a];
@@ -250,12 +275,19 @@ static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, in
         c->bbox_min[a] = origin[a];
         c->bbox_max[a] = static_cast<float>(origin[a] + static_cast<double>(n[a]) * voxel_size);
     }
-    if ((rc = build_stencils(c))) return rc;
+    if (stencils && (rc = finish_stencils(c, bits[1]))) return rc;
     c->has_volume = true;
     c->update_world_box();
     c->maj_shift = 0;  // the pooled majorant grid is rebuilt at the next launch
     VPT_CUDA(cudaDeviceSynchronize());
     return VPT_OK;
+}
+
+static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, int ny, int nz, float voxel_size,
+                                 const float origin[3]) {
+    const int rc = build_grid(c, d_dense, nx, ny, nz, voxel_size, origin);
+    if (rc) drop_stencils(c);
+    return rc;
 }
 
 int vpt_set_volume_dense(VptContext* c, const float* host, int32_t nx, int32_t ny, int32_t nz, float voxel_size,
@@ -264,8 +296,7 @@ int vpt_set_volume_dense(VptContext* c, const float* host, int32_t nx, int32_t n
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_volume_dense: bad arguments");
     int64_t total = static_cast<int64_t>(nx) * ny * nz;
     int rc;
-    drop_stencils(c);
-    if ((rc = dev_alloc(&c->d_dense, total))) return rc;
+    if ((rc = volume_alloc(c, &c->d_dense, total))) return rc;
     VPT_CUDA(cudaMemcpy(c->d_dense, host, total * sizeof(float), cudaMemcpyHostToDevice));
     return build_grid_from_dense(c, c->d_dense, nx, ny, nz, voxel_size, origin);
 }
@@ -276,8 +307,7 @@ int vpt_set_volume_dense_device(VptContext* c, const float* dev, int32_t nx, int
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_volume_dense_device: bad arguments");
     int64_t total = static_cast<int64_t>(nx) * ny * nz;
     int rc;
-    drop_stencils(c);
-    if ((rc = dev_alloc(&c->d_dense, total))) return rc;
+    if ((rc = volume_alloc(c, &c->d_dense, total))) return rc;
     VPT_CUDA(cudaMemcpy(c->d_dense, dev, total * sizeof(float), cudaMemcpyDeviceToDevice));
     return build_grid_from_dense(c, c->d_dense, nx, ny, nz, voxel_size, origin);
 }
@@ -289,8 +319,7 @@ int vpt_generate_fbm_volume(VptContext* c, int32_t n, uint32_t seed, int32_t oct
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_generate_fbm_volume: bad arguments");
     int64_t total = static_cast<int64_t>(n) * n * n;
     int rc;
-    drop_stencils(c);
-    if ((rc = dev_alloc(&c->d_dense, total))) return rc;
+    if ((rc = volume_alloc(c, &c->d_dense, total))) return rc;
     vpt::generate_fbm(c->d_dense, n, seed, octaves, lacunarity, gain, base_frequency, threshold, c->d_scratch_u32, 0);
     VPT_CUDA(cudaGetLastError());
     return build_grid_from_dense(c, c->d_dense, n, n, n, voxel_size, origin);
@@ -304,10 +333,9 @@ int vpt_generate_fbm_union(VptContext* c, int32_t n, uint32_t seed_a, uint32_t s
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_generate_fbm_union: bad arguments");
     int64_t total = static_cast<int64_t>(n) * n * n;
     int rc;
-    drop_stencils(c);
-    if ((rc = dev_alloc(&c->d_dense, total))) return rc;
+    if ((rc = volume_alloc(c, &c->d_dense, total))) return rc;
     float* second = nullptr;
-    if ((rc = dev_alloc(&second, total))) return rc;
+    if ((rc = volume_alloc(c, &second, total))) return rc;
     vpt::generate_fbm(c->d_dense, n, seed_a, octaves, lacunarity, gain, base_frequency, threshold, c->d_scratch_u32, 0);
     vpt::generate_fbm(second, n, seed_b, octaves, lacunarity, gain, base_frequency, threshold, c->d_scratch_u32, 0);
     vpt::max_into(c->d_dense, second, total, 0);
@@ -748,7 +776,7 @@ namespace vpt {
 // leaf-aligned extent starting at index `lo`, and the grid's map and boxes. Cell majorants use
 // the same apron as the dense build; the global majorant scans [index_min, index_max) of the
 // grid's index box (renderer/renderer_scene.cpp:498-509).
-int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int32_t lx, int32_t ly, int32_t lz,
+static int upload_grid(VptContextImpl* c, const std::vector<int32_t>& table, int32_t lx, int32_t ly, int32_t lz,
                        const std::vector<int32_t>& origins, const float* values, int64_t slots, const int32_t lo[3],
                        const VptNanoVdbInfo& info) {
     const int64_t cells = static_cast<int64_t>(lx) * ly * lz;
@@ -756,9 +784,9 @@ int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
     begin_volume(c);
     int32_t* d_origins = nullptr;
     int rc;
-    if ((rc = dev_alloc(&c->d_cell_maj, cells)) || (rc = dev_alloc(&c->d_leaf_table, cells)) ||
-        (rc = dev_alloc(&c->d_leaf_values, std::max<int64_t>(slots, 1) * 512)) ||
-        (rc = dev_alloc(&d_origins, std::max<int64_t>(slots, 1) * 3)))
+    if ((rc = volume_alloc(c, &c->d_cell_maj, cells)) || (rc = volume_alloc(c, &c->d_leaf_table, cells)) ||
+        (rc = volume_alloc(c, &c->d_leaf_values, std::max<int64_t>(slots, 1) * 512)) ||
+        (rc = volume_alloc(c, &d_origins, std::max<int64_t>(slots, 1) * 3)))
         return rc;
     VPT_CUDA(cudaMemcpy(c->d_leaf_table, table.data(), cells * sizeof(int32_t), cudaMemcpyHostToDevice));
     if (slots > 0) {
@@ -779,11 +807,12 @@ int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
     }
     vpt::leaf_box_max(c->d_leaf_values, d_origins, slots, box_lo, box_hi, c->d_scratch_u32, 0);
     cudaError_t e = cudaGetLastError();
-    unsigned int gmax_bits = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&gmax_bits, c->d_scratch_u32, sizeof(unsigned int), cudaMemcpyDeviceToHost);
+    const bool stencils = e == cudaSuccess && begin_stencils(c);
+    unsigned int bits[2] = {0, 0};  // global majorant, slots of the stencil copy
+    if (e == cudaSuccess) e = cudaMemcpy(bits, c->d_scratch_u32, sizeof(bits), cudaMemcpyDeviceToHost);
     dev_free(&d_origins);
     if (e != cudaSuccess) return set_error(VPT_ERR_CUDA, std::string("vpt_set_volume_nanovdb: ") + cudaGetErrorString(e));
-    std::memcpy(&c->global_majorant, &gmax_bits, sizeof(float));
+    std::memcpy(&c->global_majorant, bits, sizeof(float));
     c->active_leaves = slots;
     c->total_leaves = cells;
     // Lookups map world p to index (p - origin) * inv_voxel_size, origin being the world position
@@ -796,12 +825,20 @@ int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
         c->bbox_min[a] = static_cast<float>(info.world_min[a]);
         c->bbox_max[a] = static_cast<float>(info.world_max[a]);
     }
-    if ((rc = build_stencils(c))) return rc;
+    if (stencils && (rc = finish_stencils(c, bits[1]))) return rc;
     c->has_volume = true;
     c->update_world_box();
     c->maj_shift = 0;  // the pooled majorant grid is rebuilt at the next launch
     VPT_CUDA(cudaDeviceSynchronize());
     return VPT_OK;
+}
+
+int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int32_t lx, int32_t ly, int32_t lz,
+                       const std::vector<int32_t>& origins, const float* values, int64_t slots, const int32_t lo[3],
+                       const VptNanoVdbInfo& info) {
+    const int rc = upload_grid(c, table, lx, ly, lz, origins, values, slots, lo, info);
+    if (rc) drop_stencils(c);
+    return rc;
 }
 
 }  // namespace vpt

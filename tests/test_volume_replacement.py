@@ -61,3 +61,30 @@ r.close()
 print("ok", fake.fake_bytes())
 """, tmp_path)
     assert out.split() == ["ok", "0"]
+
+
+@pytest.mark.parametrize("kind", list(SETTERS))
+def test_replacement_reuses_the_copys_memory(tmp_path, kind):
+    """A replacement of like size (a frame of a moving cloud) allocates the volume's own arrays and
+    nothing for the copy, reads back the active leaves and the majorant and nothing else; a much smaller
+    volume does not keep the large one's copy."""
+    out = _fake_cuda.run(f"set_volume = {SETTERS[kind]}\nclouds = {2 if kind == 'union' else 1}\n" + """
+r = Renderer(8, 8)
+set_volume(r, 64)
+held = fake.fake_bytes()
+before = [fake.fake_calls(k) for k in (MALLOC, COPY, MEMINFO)]
+set_volume(r, 64)
+calls = [fake.fake_calls(k) - b for k, b in zip((MALLOC, COPY, MEMINFO), before)]
+# voxels of each cloud, active leaves, tables and leaves; copies: the voxels (or a cloud's range), the
+# active leaves, the leaf table, the majorant with the copy's size
+assert calls == [clouds + 4, clouds + 3, 0], calls
+assert fake.fake_bytes() == held
+set_volume(r, 16)
+small = fake.fake_bytes()
+r.close()
+r = Renderer(8, 8)
+set_volume(r, 16)
+assert small == fake.fake_bytes()
+print("ok")
+""", tmp_path)
+    assert out.split() == ["ok"]
