@@ -108,6 +108,10 @@ int vpt_get_rng_states(VptContext* ctx, uint64_t* host_states);
  * is stored on the device as NanoVDB-style 8^3 leaves (values ordered x<<6|y<<3|z) reached
  * through a dense leaf table; all-zero leaves are not stored. World position of voxel index
  * (i,j,k) is origin + (i,j,k) * voxel_size; the clip box is [origin, origin + n * voxel_size].
+ * Beside the leaves, the context holds a copy of the grid in which every voxel's 2x2x2 stencil
+ * lies together (eight times the leaves' bytes; one load per lookup), for the tracker with work
+ * queues, where that takes at most half of the free device memory; without it launches read the
+ * leaves, with the same results. Setting the next volume reuses the copy's memory or gives it back.
  * Replaces Scene::allocateVolumeGrid (renderer/renderer_scene.cpp:491-537), including its
  * global majorant scan over [min, max) of the index box (:498-509). */
 int vpt_set_volume_dense(VptContext* ctx, const float* host_voxels, int32_t nx, int32_t ny,
@@ -250,7 +254,9 @@ int vpt_set_surfaces(VptContext* ctx, const VptSurfaceMaterial* materials, uint3
  * world box (6 floats: min, max) the launches use. Any pointer may be NULL. */
 int vpt_get_surface_info(VptContext* ctx, uint32_t* triangles, uint32_t* bvh_nodes, uint32_t* emitters,
                          float* world_box);
-/* Removes the density volume (a surface-only scene: the reference without a density grid). */
+/* Removes the density volume (a surface-only scene: the reference without a density grid). The copy
+ * of the grid that speeds lookups up (see vpt_set_volume_dense) is given back; the leaves stay
+ * allocated for the next volume. Launches captured in a CUDA graph before are to be captured again. */
 int vpt_clear_volume(VptContext* ctx);
 
 /* Image-based environment from an RGB float image (row-major, rows = polar angle from +y).

@@ -48,25 +48,13 @@ void dev_free(T** p) {
     *p = nullptr;
 }
 
-// Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
-// for one 32-byte load per lookup. Taken only where it needs at most half of the free device memory;
-// a larger grid is traced from its leaves. A replacement of like size builds its copy in the old
-// one's memory (us per call, without a copy / with allocations of its own / so: 64^3 102 / 304 / 128,
-// 128^3 426 / 636 / 462, 200^3 649 / 1003 / 755; the rest is its two kernels); that
-// memory gives way where the new volume's arrays have no room beside it.
-void drop_stencils(vpt::VptContextImpl* c) {
-    dev_free(&c->d_st_table);
-    dev_free(&c->d_st_values);
-    c->st_table_cap = c->st_values_cap = 0;
-}
-
 // Memory for one of a volume's arrays.
 template <typename T>
 int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
     int rc = dev_alloc(p, count);
     if (rc && c->d_st_table) {
         cudaGetLastError();
-        drop_stencils(c);
+        c->release_stencils();
         rc = dev_alloc(p, count);
     }
     return rc;
@@ -75,6 +63,18 @@ int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
 }  // namespace
 
 namespace vpt {
+// Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
+// for one 32-byte load per lookup. Taken only where it needs at most half of the free device memory;
+// a larger grid is traced from its leaves. A replacement of like size builds its copy in the old
+// one's memory (us per call, without a copy / with allocations of its own / so: 64^3 102 / 304 / 128,
+// 128^3 426 / 636 / 462, 200^3 649 / 1003 / 755; the rest is its two kernels); that
+// memory gives way where the new volume's arrays have no room beside it.
+void VptContextImpl::release_stencils() {
+    dev_free(&d_st_table);
+    dev_free(&d_st_values);
+    st_table_cap = st_values_cap = 0;
+}
+
 int ctx_set_error(int code, const char* msg) { return set_error(code, msg); }
 }  // namespace vpt
 
@@ -138,8 +138,7 @@ int vpt_destroy(VptContext* c) {
     dev_free(&c->d_integral);
     dev_free(&c->d_leaf_table);
     dev_free(&c->d_leaf_values);
-    dev_free(&c->d_st_table);
-    dev_free(&c->d_st_values);
+    c->release_stencils();
     dev_free(&c->d_cell_maj);
     dev_free(&c->d_maj);
     dev_free(&c->d_jumps);
@@ -206,7 +205,7 @@ static bool begin_stencils(VptContextImpl* c) {
         c->st_table_cap = 0;
         if (dev_alloc(&c->d_st_table, 2 * cells)) {
             cudaGetLastError();  // traced from the leaves
-            drop_stencils(c);
+            c->release_stencils();
             return false;
         }
         c->st_table_cap = 2 * cells;
@@ -227,7 +226,7 @@ static int finish_stencils(VptContextImpl* c, unsigned int slots) {
         VPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
         if (values * sizeof(float) > free_bytes / 2 || dev_alloc(&c->d_st_values, values)) {
             cudaGetLastError();
-            drop_stencils(c);
+            c->release_stencils();
             return VPT_OK;
         }
         c->st_values_cap = values;
@@ -286,7 +285,7 @@ static int build_grid(VptContext* c, const float* d_dense, int nx, int ny, int n
 static int build_grid_from_dense(VptContext* c, const float* d_dense, int nx, int ny, int nz, float voxel_size,
                                  const float origin[3]) {
     const int rc = build_grid(c, d_dense, nx, ny, nz, voxel_size, origin);
-    if (rc) drop_stencils(c);
+    if (rc) c->release_stencils();
     return rc;
 }
 
@@ -837,7 +836,7 @@ int upload_sparse_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
                        const std::vector<int32_t>& origins, const float* values, int64_t slots, const int32_t lo[3],
                        const VptNanoVdbInfo& info) {
     const int rc = upload_grid(c, table, lx, ly, lz, origins, values, slots, lo, info);
-    if (rc) drop_stencils(c);
+    if (rc) c->release_stencils();
     return rc;
 }
 

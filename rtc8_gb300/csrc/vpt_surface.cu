@@ -526,6 +526,7 @@ int vpt_get_surface_info(VptContext* c, uint32_t* triangles, uint32_t* bvh_nodes
 int vpt_clear_volume(VptContext* c) {
     if (!c) return vpt::fail(VPT_ERR_INVALID_ARGUMENT, "vpt_clear_volume: null context");
     c->has_volume = false;
+    c->release_stencils();
     c->update_world_box();
     return VPT_OK;
 }

@@ -88,3 +88,20 @@ assert small == fake.fake_bytes()
 print("ok")
 """, tmp_path)
     assert out.split() == ["ok"]
+
+
+def test_cleared_volume_gives_the_copy_back(tmp_path):
+    out = _fake_cuda.run("""
+r = Renderer(8, 8)
+empty = fake.fake_bytes()
+r.set_volume_dense(np.ones((64, 64, 64), np.float32), 1 / 64, [-0.5] * 3)
+r.clear_volume()
+# what stays: dense voxels, two tables, one leaf
+assert fake.fake_bytes() - empty == 4 * 64 ** 3 + 2 * 4 * 8 ** 3 + 4 * 512, fake.fake_bytes() - empty
+r.set_volume_dense(np.ones((64, 64, 64), np.float32), 1 / 64, [-0.5] * 3)
+r.set_frame(frame_params(C1))
+r.launch_plain(1)
+r.close()
+print("ok", fake.fake_bytes())
+""", tmp_path)
+    assert out.split() == ["ok", "0"]
