@@ -132,7 +132,8 @@ int vpt_generate_fbm_union(VptContext* ctx, int32_t n, uint32_t seed_a, uint32_t
 /* Copies the dense voxel values of the last generated/uploaded volume to the host (n^3 floats);
  * only valid until the next volume call. */
 int vpt_download_volume_dense(VptContext* ctx, float* host_voxels);
-/* Grid statistics: active leaves, total leaves, global majorant, device bytes of the grid. */
+/* Grid statistics: active leaves, total leaves, global majorant, device bytes of the grid (leaves,
+ * tables and, where it is held, the stencil copy; not the dense voxels). */
 int vpt_get_volume_info(VptContext* ctx, int64_t* active_leaves, int64_t* total_leaves,
                         float* global_majorant, int64_t* grid_bytes);
 /* Per-cell majorants (one per 8^3 leaf cell, max over the cell's voxels plus a one-voxel

@@ -357,7 +357,8 @@ int vpt_get_volume_info(VptContext* c, int64_t* active, int64_t* total, float* g
     if (active) *active = c->active_leaves;
     if (total) *total = c->total_leaves;
     if (gmaj) *gmaj = c->global_majorant;
-    if (bytes) *bytes = c->active_leaves * 512 * 4 + c->total_leaves * 8;
+    // Leaves, leaf table and cell majorants; the stencil copy's table (with its slots' cells) and values.
+    if (bytes) *bytes = c->active_leaves * 512 * 4 + c->total_leaves * 8 + (c->st_table_cap + c->st_values_cap) * 4;
     return VPT_OK;
 }
 

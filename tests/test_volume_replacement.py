@@ -105,3 +105,25 @@ r.close()
 print("ok", fake.fake_bytes())
 """, tmp_path)
     assert out.split() == ["ok", "0"]
+
+
+def test_volume_info_counts_the_copy(tmp_path):
+    """The reported bytes are those held for the grid, with the copy and, where there is no room for it,
+    without."""
+    out = _fake_cuda.run("""
+for room in (1 << 40, 0):
+    fake.fake_limit(1 << 40)
+    r = Renderer(8, 8)
+    r.set_volume_dense(np.ones((64, 64, 64), np.float32), 1 / 64, [-0.5] * 3)
+    r.clear_volume()
+    if not room:
+        fake.fake_limit(fake.fake_bytes() + 4 * 8 ** 3)  # the volume's arrays again and the builder's list of cells
+    empty = fake.fake_bytes() - (4 * 64 ** 3 + 2 * 4 * 8 ** 3 + 4 * 512)
+    r.set_volume_dense(np.ones((64, 64, 64), np.float32), 1 / 64, [-0.5] * 3)
+    held = fake.fake_bytes() - empty - 4 * 64 ** 3 - 4 * 512  # without the voxels and the one leaf that no active leaf fills
+    assert r.volume_info()["grid_bytes"] == held, (room, r.volume_info(), held)
+    assert (held > 2 * 4 * 8 ** 3) == bool(room)
+    r.close()
+print("ok")
+""", tmp_path)
+    assert out.split() == ["ok"]
