@@ -111,13 +111,20 @@ int vpt_get_rng_states(VptContext* ctx, uint64_t* host_states);
  * Beside the leaves, the context holds a copy of the grid in which every voxel's 2x2x2 stencil
  * lies together (eight times the leaves' bytes; one load per lookup), for the tracker with work
  * queues, where that takes at most half of the free device memory; without it launches read the
- * leaves, with the same results. Setting the next volume reuses the copy's memory or gives it back.
+ * leaves, with the same results (vpt_set_stencil_limit bounds it or switches it off). Setting the
+ * next volume reuses the copy's memory or gives it back.
  * Replaces Scene::allocateVolumeGrid (renderer/renderer_scene.cpp:491-537), including its
  * global majorant scan over [min, max) of the index box (:498-509). */
 int vpt_set_volume_dense(VptContext* ctx, const float* host_voxels, int32_t nx, int32_t ny,
                          int32_t nz, float voxel_size, const float origin[3]);
 int vpt_set_volume_dense_device(VptContext* ctx, const float* dev_voxels, int32_t nx, int32_t ny,
                                 int32_t nz, float voxel_size, const float origin[3]);
+/* Device bytes the stencil copy of the grid may take: -1 (the default) = half of the memory that is
+ * free when it is made, 0 = no copy (for callers who need the memory, and for the wavefront
+ * tracker and leaf staging, which read the leaves). Holds for the volumes set from then on; a copy held
+ * beyond the limit is given back at once, and launches captured in a CUDA graph before are then to
+ * be captured again. */
+int vpt_set_stencil_limit(VptContext* ctx, int64_t max_bytes);
 /* Seeded fBm value-noise volume generated on the device (octaves, lacunarity, gain, base
  * frequency in lattice cells across the grid). Values are remapped so min..max -> [0,1];
  * with threshold > 0 they become max(0, (r - threshold) / (1 - threshold)). */

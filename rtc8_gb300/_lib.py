@@ -128,6 +128,7 @@ _VPT = {
                                               c_float_p]),
     "vpt_generate_fbm_volume": (C.c_int, [C.c_void_p, C.c_int32, C.c_uint32, C.c_int32, C.c_float, C.c_float, C.c_float,
                                           C.c_float, C.c_float, c_float_p]),
+    "vpt_set_stencil_limit": (C.c_int, [C.c_void_p, C.c_int64]),
     "vpt_download_volume_dense": (C.c_int, [C.c_void_p, c_float_p]),
     "vpt_get_volume_info": (C.c_int, [C.c_void_p, c_i64_p, c_i64_p, c_float_p, c_i64_p]),
     "vpt_download_cell_majorants": (C.c_int, [C.c_void_p, c_float_p]),

@@ -64,8 +64,8 @@ int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
 
 namespace vpt {
 // Stencil copy of the leaf grid (Grid::st_table, st_values): eight times the bytes of the leaves,
-// for one 32-byte load per lookup. Taken only where it needs at most half of the free device memory;
-// a larger grid is traced from its leaves. A replacement of like size builds its copy in the old
+// for one 32-byte load per lookup. Taken only where it needs at most half of the free device memory
+// and no more than the context's limit; a larger grid is traced from its leaves. A replacement of like size builds its copy in the old
 // one's memory (us per call, without a copy / with allocations of its own / so: 64^3 102 / 304 / 128,
 // 128^3 426 / 636 / 462, 200^3 649 / 1003 / 755; the rest is its two kernels); that
 // memory gives way where the new volume's arrays have no room beside it.
@@ -197,10 +197,19 @@ static void begin_volume(VptContextImpl* c) {
     c->update_world_box();
 }
 
+// Whether a copy of so many table entries and values keeps the context's limit.
+static bool stencils_allowed(const VptContextImpl* c, int64_t entries) {
+    return c->st_limit < 0 || entries * 4 <= c->st_limit;
+}
+
 // The first half, once the leaves and their table are in place: the cells' slots (and behind them, in
 // the same array, the slots' cells), their count in d_scratch_u32[1]. False where there is no room.
 static bool begin_stencils(VptContextImpl* c) {
     const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
+    if (!stencils_allowed(c, 2 * cells + 4096)) {
+        c->release_stencils();
+        return false;
+    }
     if (c->st_table_cap < 2 * cells || c->st_table_cap > 4 * cells) {
         c->st_table_cap = 0;
         if (dev_alloc(&c->d_st_table, 2 * cells)) {
@@ -219,7 +228,11 @@ static bool begin_stencils(VptContextImpl* c) {
 static int finish_stencils(VptContextImpl* c, unsigned int slots) {
     const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
     const int64_t values = static_cast<int64_t>(std::max(slots, 1u)) * 4096;
-    if (c->st_values_cap < values || c->st_values_cap > 2 * values) {
+    if (!stencils_allowed(c, 2 * cells + values)) {
+        c->release_stencils();
+        return VPT_OK;
+    }
+    if (c->st_values_cap < values || c->st_values_cap > 2 * values || !stencils_allowed(c, c->st_table_cap + c->st_values_cap)) {
         c->st_values_cap = 0;
         dev_free(&c->d_st_values);
         size_t free_bytes = 0, total_bytes = 0;
@@ -479,6 +492,13 @@ int vpt_set_leaf_staging(VptContext* c, int32_t min_lanes) {
     if (!c || min_lanes < 0 || min_lanes > 32)
         return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_leaf_staging: min_lanes must lie in [0, 32]");
     c->leaf_stage_min = min_lanes;
+    return VPT_OK;
+}
+
+int vpt_set_stencil_limit(VptContext* c, int64_t max_bytes) {
+    if (!c || max_bytes < -1) return set_error(VPT_ERR_INVALID_ARGUMENT, "vpt_set_stencil_limit: bad arguments");
+    c->st_limit = max_bytes;
+    if (!stencils_allowed(c, c->st_table_cap + c->st_values_cap)) c->release_stencils();
     return VPT_OK;
 }
 

@@ -73,6 +73,7 @@ struct VptContextImpl {
     int32_t* d_st_table = nullptr;   // stencil copy of the grid (Grid::st_table); absent = not built
     float* d_st_values = nullptr;
     int64_t st_table_cap = 0, st_values_cap = 0;  // their sizes in entries
+    int64_t st_limit = -1;           // bytes they may take, -1 = half of the free memory (vpt_set_stencil_limit)
     void release_stencils();
     float* d_cell_maj = nullptr;
     float* d_maj = nullptr;          // majorant grid of the DDA (pooled cells)

@@ -116,6 +116,11 @@ class Renderer:
         check(self.lib.vpt_download_volume_dense(self.ctx, ptr(out, C.c_float)), "vpt_download_volume_dense")
         return out
 
+    def set_stencil_limit(self, max_bytes: int = -1) -> None:
+        """Device bytes the stencil copy of the grid may take (-1 = half of the free memory, 0 = no copy);
+        see vpt_set_stencil_limit."""
+        check(self.lib.vpt_set_stencil_limit(self.ctx, max_bytes), "vpt_set_stencil_limit")
+
     def volume_info(self) -> dict:
         a, t, b = C.c_int64(), C.c_int64(), C.c_int64()
         m = C.c_float()

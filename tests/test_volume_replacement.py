@@ -127,3 +127,37 @@ for room in (1 << 40, 0):
 print("ok")
 """, tmp_path)
     assert out.split() == ["ok"]
+
+
+def test_stencil_limit(tmp_path):
+    """0 switches the copy off, a limit below its size too, -1 back on; lowering the limit gives a held
+    copy back at once; launches go on."""
+    out = _fake_cuda.run("""
+r = Renderer(8, 8)
+r.set_frame(frame_params(C1))
+def put(n=64):
+    r.set_volume_dense(np.ones((n, n, n), np.float32), 1 / n, [-0.5] * 3)
+    r.launch_plain(1)
+    return r.volume_info()["grid_bytes"]
+plain, copy = 2 * 4 * 8 ** 3, 2 * 4 * 9 ** 3 + 4 * 4096   # tables; the copy's tables and one slot
+assert put() == plain + copy
+for limit, held in ((0, 0), (copy - 1, 0), (copy, copy), (-1, copy), (1 << 40, copy)):
+    r.set_stencil_limit(limit)
+    assert put() == plain + held, limit
+before = fake.fake_bytes()
+r.set_stencil_limit(copy - 1)
+assert fake.fake_bytes() == before - copy and r.volume_info()["grid_bytes"] == plain
+r.launch_plain(1)
+# a copy in a larger one's memory keeps the limit too
+r.set_stencil_limit(-1)
+put(64)
+small = 2 * 4 * 8 ** 3 + 4 * 4096
+r.set_stencil_limit(copy)
+assert put(56) == 2 * 4 * 7 ** 3 + copy
+r.set_stencil_limit(small)
+assert put(56) == 2 * 4 * 7 ** 3 + small
+assert failed(lambda: r.set_stencil_limit(-2))
+r.close()
+print("ok", fake.fake_bytes())
+""", tmp_path)
+    assert out.split() == ["ok", "0"]
