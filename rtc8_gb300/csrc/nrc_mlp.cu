@@ -1309,6 +1309,7 @@ struct NrcHandle {
     uint32_t* train_features = nullptr;      // hash grid only: features of a training step's records
     std::shared_ptr<WorkspacePool> pool;  // hash grid only; null = batches run the fused kernels
     uint64_t steps = 0;
+    bool accumulating = false;  // a step's gradient launch has no update behind it (a launch failed)
     int total_params() const { return ly.nparams + ly.grid_params; }
     const uint32_t* grid_words(bool train) const {
         return reinterpret_cast<const uint32_t*>(train ? grid_train : grid_infer);
@@ -1592,6 +1593,11 @@ int nrc_train(NrcHandle* h, void* stream, const float* in, const float* target, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const NetLayout& ly = h->ly;
     const uint32_t tiles = (n + kTile - 1) / kTile;
+    if (h->accumulating) {  // Adam clears what it has read: here it did not run
+        NRC_CUDA(cudaMemsetAsync(h->grad, 0, h->total_params() * sizeof(float), s));
+        NRC_CUDA(cudaMemsetAsync(h->loss, 0, sizeof(float), s));
+    }
+    h->accumulating = true;
     ++h->steps;
     const NrcConfig& c = h->cfg;
     const float c1 = 1.0f - std::pow(c.beta1, static_cast<float>(h->steps));
@@ -1631,6 +1637,7 @@ int nrc_train(NrcHandle* h, void* stream, const float* in, const float* target, 
     }
     NRC_CUDA(cudaLaunchKernelEx(shape((ly.nparams + 255) / 256 + (ly.grid_params + 1023) / 1024, 256, 0), adam_kernel, ly,
                                 adam));
+    h->accumulating = false;
     if (loss_out) {
         NRC_CUDA(cudaMemcpyAsync(loss_out, h->loss_out, sizeof(float), cudaMemcpyDeviceToHost, s));
         NRC_CUDA(cudaStreamSynchronize(s));
