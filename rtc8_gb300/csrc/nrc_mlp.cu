@@ -1301,8 +1301,9 @@ struct NrcHandle {
     int num_sms = 0;
     int infer_groups = 1;  // 128-row tiles in flight per inference CTA
     float *w = nullptr, *m = nullptr, *v = nullptr, *ema = nullptr;
-    float *grad = nullptr, *loss = nullptr;          // accumulators of a step, zero between steps
-    float *grad_out = nullptr, *loss_out = nullptr;  // the last step's
+    // One allocation (grad): a step's accumulators, zero between steps, then the last step's values.
+    float *grad = nullptr, *loss = nullptr;
+    float *grad_out = nullptr, *loss_out = nullptr;
     uint8_t *blob_train = nullptr, *blob_infer = nullptr;
     __half *grid_train = nullptr, *grid_infer = nullptr;  // FP16 hash-grid tables (hash grid only)
     unsigned int* err = nullptr;
@@ -1435,19 +1436,22 @@ int nrc_create(const NrcConfig* cfg, NrcHandle** out) {
     cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, dev);
     const int np = h->total_params();
     const int ng = std::max(h->ly.grid_params, 2);
+    const size_t accumulators = 2 * (static_cast<size_t>(np) + 4);  // np is a multiple of 4: all stay 16-byte aligned
     int rc;
-    if ((rc = alloc(&h->w, np)) || (rc = alloc(&h->m, np)) || (rc = alloc(&h->v, np)) || (rc = alloc(&h->grad, np)) ||
-        (rc = alloc(&h->grad_out, np)) || (rc = alloc(&h->loss_out, 1)) || (rc = alloc(&h->ema, np)) || (rc = alloc(&h->loss, 1)) || (rc = alloc(&h->blob_train, h->ly.blob_bytes)) ||
+    if ((rc = alloc(&h->w, np)) || (rc = alloc(&h->m, np)) || (rc = alloc(&h->v, np)) || (rc = alloc(&h->grad, accumulators)) ||
+        (rc = alloc(&h->ema, np)) || (rc = alloc(&h->blob_train, h->ly.blob_bytes)) ||
         (rc = alloc(&h->blob_infer, h->ly.blob_bytes)) || (rc = alloc(&h->grid_train, ng)) ||
         (rc = alloc(&h->grid_infer, ng)) || (rc = alloc(&h->err, 1))) {
         nrc_destroy(h);
         return rc;
     }
+    h->loss = h->grad + np;
+    h->grad_out = h->loss + 4;
+    h->loss_out = h->grad_out + np;
     const std::vector<float> w = initial_weights(h->ly, np, cfg->seed);
     if (cudaMemcpy(h->w, w.data(), np * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(h->m, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->v, 0, np * sizeof(float)) != cudaSuccess ||
-        cudaMemset(h->grad, 0, np * sizeof(float)) != cudaSuccess ||
-        cudaMemset(h->grad_out, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->loss, 0, sizeof(float)) != cudaSuccess ||
+        cudaMemset(h->grad, 0, accumulators * sizeof(float)) != cudaSuccess ||
         cudaMemset(h->ema, 0, np * sizeof(float)) != cudaSuccess || cudaMemset(h->err, 0, sizeof(unsigned int)) != cudaSuccess) {
         nrc_destroy(h);
         return fail(NRC_ERR_CUDA, "nrc_create: initial upload failed");
@@ -1501,9 +1505,6 @@ int nrc_destroy(NrcHandle* h) {
     cudaFree(h->v);
     cudaFree(h->grad);
     cudaFree(h->ema);
-    cudaFree(h->loss);
-    cudaFree(h->grad_out);
-    cudaFree(h->loss_out);
     cudaFree(h->train_features);
     cudaFree(h->blob_train);
     cudaFree(h->blob_infer);
@@ -1594,8 +1595,7 @@ int nrc_train(NrcHandle* h, void* stream, const float* in, const float* target, 
     const NetLayout& ly = h->ly;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     if (h->accumulating) {  // Adam clears what it has read: here it did not run
-        NRC_CUDA(cudaMemsetAsync(h->grad, 0, h->total_params() * sizeof(float), s));
-        NRC_CUDA(cudaMemsetAsync(h->loss, 0, sizeof(float), s));
+        NRC_CUDA(cudaMemsetAsync(h->grad, 0, (h->total_params() + 1) * sizeof(float), s));  // and the loss
     }
     h->accumulating = true;
     ++h->steps;
