@@ -97,6 +97,11 @@ uint64_t nrc_step_count(NrcHandle* h);
 /* Error bits of bounded device-side waits (tensor-core completion) since the last call; 0 = ok. */
 uint32_t nrc_device_errors(NrcHandle* h);
 
+/* Limits, in polls, of the kernels' waits for a copy and for a tensor-core product, for the calls from
+ * now on (larger values: the default, 2^18). A kernel whose wait gives up sets the error word, waits for
+ * what it started, writes no output (a training step: no gradient of that part) and ends. For testing that path: a
+ * limit of 0 makes every such wait give up. */
+int nrc_selftest_wait_limits(NrcHandle* h, uint32_t copy_polls, uint32_t product_polls);
 /* Tensor-core self test: D = A * B^T for A (128 x 64) and B (64 x 64) given as FP32 host arrays
  * (rounded to FP16), with the operands staged in shared memory K-major (0) or MN-major (1);
  * writes D (128 x 64, FP32) to host memory. Checks the shared-memory descriptor layouts the

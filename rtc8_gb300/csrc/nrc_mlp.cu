@@ -81,6 +81,7 @@ struct NetLayout {
     uint32_t grid_off[kGridLevels], grid_size[kGridLevels], grid_res[kGridLevels];
     float grid_scale[kGridLevels];
     uint32_t grid_hashed;
+    uint32_t copy_polls, product_polls;  // limits of the kernels' waits (mbar_wait)
 };
 
 // Level geometry of the hash grid: scale 16 * 2^l - 1, resolution ceil(scale) + 1, table size
@@ -125,6 +126,7 @@ NetLayout make_layout(int enc, int hidden, int out_act, float loss_scale) {
     l.blob_bytes = bo;
     l.out_act = out_act;
     l.loss_scale = loss_scale;
+    l.copy_polls = l.product_polls = kWaitPolls;
     return l;
 }
 
@@ -590,9 +592,9 @@ __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const Ne
         bulk_load(s_table, grid + ly.grid_off[lv], ly.grid_size[lv] * 4, &s_bar);
     }
     __syncthreads();
-    if (!__syncthreads_and(mbar_wait(&s_bar, 0))) {
+    if (!__syncthreads_and(mbar_wait(&s_bar, 0, ly.copy_polls))) {
         if (threadIdx.x == 0) atomicOr(err, kErrTimeout);
-        mbar_wait(&s_bar, 0);  // again bounded: the copy must not land in another CTA's shared memory
+        mbar_wait(&s_bar, 0);
         return;
     }
     uint32_t* const out = features + static_cast<size_t>(lv) * stride;
@@ -676,7 +678,7 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
     const uint32_t first = g * gridDim.x + blockIdx.x;
     load_query(in, idx, first * kTile + gt, n, q);
     load_features(first * kTile + gt);
-    ok = named_sync_and(bar_id, kTile, mbar_wait(s_wbar, 0));
+    ok = named_sync_and(bar_id, kTile, mbar_wait(s_wbar, 0, ly.copy_polls));
     for (uint32_t tile = first; tile < ntiles && ok; tile += stride) {
         const uint32_t row = tile * kTile + gt;
         if constexpr (FEAT)
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
 
             // Each thread waits for the product itself; the group decides whether to go on at the
             // barrier after the epilogue (one barrier per layer).
-            ok = mbar_wait(s_bar + g, phase);
+            ok = mbar_wait(s_bar + g, phase, ly.product_polls);
             phase ^= 1;
             __syncwarp();
             tc_fence_after();
@@ -753,7 +755,11 @@ __global__ void __launch_bounds__(kTile* G, 1) mlp_infer_kernel(const NetLayout 
             }
         }
     }
-    if (!ok && gt == 0) atomicOr(err, kErrTimeout);
+    if (!ok) {  // the weights, and the last product that was issued (none: the wait's phase is past)
+        mbar_wait(s_wbar, 0);
+        mbar_wait(s_bar + g, phase ^ 1);
+        if (gt == 0) atomicOr(err, kErrTimeout);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -829,7 +835,7 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayou
     }
     fence_async_smem();
     tc_fence_before();
-    bool ok = __syncthreads_and(tid != 0 || mbar_wait(s_bar + 3, 0));
+    bool ok = __syncthreads_and(tid != 0 || mbar_wait(s_bar + 3, 0, ly.copy_polls));
     tc_fence_after();
     // Not before this CTA holds its tensor memory: CTAs of the next step must not take it first.
     grid_launch_dependents();
@@ -845,7 +851,7 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayou
             mma_commit(s_bar);
         }
         // Each thread waits for the product itself; the block decides at the barrier after the epilogue.
-        ok = mbar_wait(s_bar, phase);
+        ok = mbar_wait(s_bar, phase, ly.product_polls);
         phase ^= 1;
         __syncwarp();
         tc_fence_after();
@@ -923,12 +929,13 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayou
     };
     // The weight gradients' products complete one or two layers ahead of their reduction, so each
     // accumulator has its own mbarrier (a wait on the parity of a phase must not miss the next one).
-    uint32_t phase_w = 0;  // bit b: accumulator b
+    uint32_t phase_w = 0;  // bit b: accumulator b; kLate: a wait for one of them gave up
+    constexpr uint32_t kLate = 4;
     if (ok && tid == 0) issue_backward(L - 1);
     for (int j = L - 1; j >= 0 && ok; --j) {
         const bool chain = j > 0 || hash;
         if (chain) {
-            ok = mbar_wait(s_bar, phase);
+            ok = mbar_wait(s_bar, phase, ly.product_polls) && phase_w < kLate;
             phase ^= 1;
             __syncwarp();
             tc_fence_after();
@@ -950,14 +957,19 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayou
             tc_fence_before();
             fence_async_smem();
             ok = __syncthreads_and(ok);
-            if (!ok) break;
+            if (!ok) {
+                phase_w ^= 1u << (j & 1);  // issued, left to the wait below
+                break;
+            }
             if (tid == 0) issue_backward(j - 1);
         }
         // Weight-gradient rows: TMEM lane = output feature. The TMEM load is warp-collective, so
-        // every lane of a warp that holds gradient rows takes part; only real rows are reduced.
-        const bool done = mbar_wait(s_bar + 1 + (j & 1), (phase_w >> (j & 1)) & 1u);
+        // every lane of a warp that holds gradient rows takes part (the warp goes on or gives up as
+        // one); only real rows are reduced.
+        const bool done =
+            __all_sync(0xffffffffu, mbar_wait(s_bar + 1 + (j & 1), (phase_w >> (j & 1)) & 1u, ly.product_polls));
         phase_w ^= 1u << (j & 1);
-        __syncwarp();
+        if (!done) phase_w |= kLate;
         tc_fence_after();
         const int out_real = j == L - 1 ? 3 : ly.out[j], N_in = ly.in[j];
         if (warp * 32 < out_real && done) {
@@ -982,9 +994,13 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const NetLayou
             if (row < n && ok) grid_backward(ly, q, wg * 8, d, grad + ly.nparams);
         }
         tc_fence_before();
-        if (!done) atomicOr(err, kErrTimeout);
     }
-    if (!ok) atomicOr(err, kErrTimeout);
+    if (!ok || phase_w >= kLate) {  // the weights and the last product issued on each barrier
+        if (tid == 0) mbar_wait(s_bar + 3, 0);
+        mbar_wait(s_bar, phase ^ 1);
+        for (int b = 0; b < 2; ++b) mbar_wait(s_bar + 1 + b, ((phase_w >> b) & 1u) ^ 1u);
+        atomicOr(err, kErrTimeout);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1165,7 +1181,10 @@ __global__ void mma_rate_kernel(int n, uint32_t count, long long* __restrict__ o
             for (int ks = 0; ks < 4; ++ks) mma_f16(d, ad + 16 * ks, bd + 16 * ks, idesc, (i > 0 || ks > 0) ? 1u : 0u);
         }
         mma_commit(bar);
-        if (!mbar_wait(bar, 0)) atomicOr(err, kErrTimeout);
+        if (!mbar_wait(bar, 0)) {
+            atomicOr(err, kErrTimeout);
+            mbar_wait(bar, 0);
+        }
         out[0] = clock64() - t0;
     }
     tc_fence_before();
@@ -1228,8 +1247,9 @@ __global__ void selftest_kernel(const float* __restrict__ A, const float* __rest
             tmem_wait_ld();
             for (int i = 0; i < 16; ++i) D[tid * N + c * 16 + i] = v[i];
         }
-    } else if (tid == 0) {
-        atomicOr(err, kErrTimeout);
+    } else {
+        mbar_wait(bar, 0);
+        if (tid == 0) atomicOr(err, kErrTimeout);
     }
     tc_fence_before();
     __syncthreads();
@@ -1705,6 +1725,13 @@ uint32_t nrc_device_errors(NrcHandle* h) {
     if (cudaMemcpy(&e, h->err, sizeof(e), cudaMemcpyDeviceToHost) != cudaSuccess) return 0xffffffffu;
     cudaMemset(h->err, 0, sizeof(unsigned int));
     return e;
+}
+
+int nrc_selftest_wait_limits(NrcHandle* h, uint32_t copy_polls, uint32_t product_polls) {
+    if (!h) return fail(NRC_ERR_INVALID_ARGUMENT, "null handle");
+    h->ly.copy_polls = std::min(copy_polls, kWaitPolls);
+    h->ly.product_polls = std::min(product_polls, kWaitPolls);
+    return NRC_OK;
 }
 
 int nrc_selftest_mma_rate(int32_t n, uint32_t count, double* cycles_per_mma) {

@@ -144,9 +144,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after `limit` polls (a poll suspends the thread for up to 4 us: about a
-// second) and returns false, so a kernel can record an error and leave instead of hanging.
-__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t limit = 1u << 18) {
+// Bounded wait: gives up after `limit` polls (how long a poll suspends the thread is the hardware's
+// choice) and returns false, so a kernel can record an error and leave instead of hanging. Before it
+// leaves it waits once more, with kWaitPolls, for what it started: a copy or a product that is still
+// under way must not reach shared or tensor memory that another CTA has been given.
+constexpr uint32_t kWaitPolls = 1u << 18;
+__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t limit = kWaitPolls) {
     for (uint32_t i = 0; i < limit; ++i)
         if (mbar_try_wait(mbar, parity)) return true;
     return false;

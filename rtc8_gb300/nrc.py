@@ -135,6 +135,15 @@ class NeuralRadianceCache:
         return int(self.lib.nrc_device_errors(self.h))
 
 
+WAIT_POLLS = 1 << 18  # default limit of the kernels' waits
+
+
+def selftest_wait_limits(cache: NeuralRadianceCache, copy_polls: int = WAIT_POLLS, product_polls: int = WAIT_POLLS) -> None:
+    """nrc_selftest_wait_limits: after how many polls the cache's kernels give up a wait for a copy or
+    a tensor-core product."""
+    _check(cache.lib.nrc_selftest_wait_limits(cache.h, copy_polls, product_polls), "nrc_selftest_wait_limits")
+
+
 def selftest_mma_rate(n: int, count: int = 1024) -> float:
     """nrc_selftest_mma_rate: SM cycles per back-to-back M = 128 x N = n x K = 16 FP16 MMA issued by
     one thread (the rate the MLP kernels' layer shapes can reach)."""
