@@ -8,8 +8,7 @@ costs one graph launch. The device frame counters of each context advance inside
 every replay renders new samples. Branches of the graph run concurrently, so one scene's launch
 tail overlaps the next scene's work.
 
-The autotuner picks per scene the tracker's launch shape (CTAs per SM and the warp park
-threshold) by timing a short launch of each candidate.
+The autotuner picks per scene the tracker's CTAs per SM by timing a short launch of each candidate.
 """
 from __future__ import annotations
 
@@ -21,9 +20,10 @@ import numpy as np
 from .configs import C1, SceneConfig, VolumeSpec
 from .renderer import Renderer, setup_scene
 
-# Launch shapes the autotuner tries: (CTAs per SM, park threshold); 0 = the defaults. The batch's
+# Launch shapes the autotuner tries: (CTAs per SM, park threshold); 0 = the defaults (six CTAs fit). The
+# tracker with work queues has no park threshold; with leaf staging a caller may try some. The batch's
 # launches run CTAs of 128 threads (BATCH_THREADS), so that concurrent launches share an SM.
-LAUNCH_CANDIDATES = [(0, 0), (0, 16), (0, 28), (6, 24), (5, 24)]
+LAUNCH_CANDIDATES = [(0, 0), (5, 0), (4, 0), (3, 0)]
 BATCH_THREADS = 128
 
 
@@ -56,7 +56,7 @@ class SceneBatch:
         for cfg in self.configs:
             r = Renderer(cfg.width, cfg.height)
             setup_scene(r, cfg)
-            # The batch step is one CUDA graph: its launches are the persistent megakernel (the
+            # The batch step is one CUDA graph: its launches are the persistent tracker's (the
             # wavefront tracer issues its passes from the host and cannot be captured).
             r.set_tracker(0)
             r.set_launch_shape(0, BATCH_THREADS, 0)
@@ -103,8 +103,9 @@ class SceneBatch:
             r.set_launch_shape(best[1], BATCH_THREADS, best[2])
             r.reset_accumulation()
             self.shapes[i] = (best[1], best[2])
-            report.append({"scene": self.configs[i].name, "ctas_per_sm": best[1], "park_threshold": best[2],
-                           "ms_per_launch": best[0], "spp": spp})
+            report.append({"scene": self.configs[i].name, "ctas_per_sm": best[1], "ms_per_launch": best[0], "spp": spp})
+            if best[2]:
+                report[-1]["park_threshold"] = best[2]
         self.graph = None  # launch shapes are part of the captured launches
         return report
 
