@@ -38,7 +38,10 @@ int dev_alloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) return VPT_OK;
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
-    if (e != cudaSuccess) return set_error(VPT_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next launch as well
+        return set_error(VPT_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     return VPT_OK;
 }
 
@@ -53,7 +56,6 @@ template <typename T>
 int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
     int rc = dev_alloc(p, count);
     if (rc && c->d_st_table) {
-        cudaGetLastError();
         c->release_stencils();
         rc = dev_alloc(p, count);
     }
@@ -213,8 +215,7 @@ static bool begin_stencils(VptContextImpl* c) {
     if (c->st_table_cap < 2 * cells || c->st_table_cap > 4 * cells) {
         c->st_table_cap = 0;
         if (dev_alloc(&c->d_st_table, 2 * cells)) {
-            cudaGetLastError();  // traced from the leaves
-            c->release_stencils();
+            c->release_stencils();  // traced from the leaves
             return false;
         }
         c->st_table_cap = 2 * cells;

@@ -14,6 +14,7 @@ std::map<void*, size_t> g_live;  // device allocations
 size_t g_bytes = 0, g_limit = static_cast<size_t>(1) << 40;
 int g_fail[5] = {0, 0, 0, 0, 0};  // calls of a kind until they fail, 0 = none fails
 int g_calls[5] = {0, 0, 0, 0, 0};
+cudaError_t g_last = cudaSuccess;  // what cudaGetLastError reports once
 
 bool fails(int kind) {
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -23,9 +24,9 @@ bool fails(int kind) {
     return false;
 }
 cudaError_t take(void** p, size_t bytes) {
-    if (fails(0)) return cudaErrorMemoryAllocation;
+    if (fails(0)) return g_last = cudaErrorMemoryAllocation;
     std::lock_guard<std::mutex> lock(g_mutex);
-    if (g_bytes + bytes > g_limit) return cudaErrorMemoryAllocation;
+    if (g_bytes + bytes > g_limit) return g_last = cudaErrorMemoryAllocation;
     *p = std::calloc(1, bytes ? bytes : 1);
     g_live[*p] = bytes;
     g_bytes += bytes;
@@ -42,7 +43,7 @@ cudaError_t give(void* p) {
     return cudaSuccess;
 }
 cudaError_t launch() {
-    return fails(3) ? cudaErrorLaunchOutOfResources : cudaSuccess;
+    return fails(3) ? g_last = cudaErrorLaunchOutOfResources : cudaSuccess;
 }
 }  // namespace
 
@@ -73,13 +74,13 @@ cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { ret
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t bytes, cudaMemPool_t, cudaStream_t) { return take(p, bytes); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return give(p); }
 cudaError_t cudaMemGetInfo(size_t* free_bytes, size_t* total) {
-    if (fails(2)) return cudaErrorUnknown;
+    if (fails(2)) return g_last = cudaErrorInvalidValue;
     *free_bytes = g_limit > g_bytes ? g_limit - g_bytes : 0;
     *total = g_limit;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* dst, const void* src, size_t bytes, cudaMemcpyKind) {
-    if (fails(1)) return cudaErrorUnknown;
+    if (fails(1)) return g_last = cudaErrorInvalidValue;
     std::memcpy(dst, src, bytes);
     return cudaSuccess;
 }
@@ -88,7 +89,7 @@ cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpy
 }
 cudaError_t cudaMemcpyToSymbol(const void*, const void*, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
 cudaError_t cudaMemset(void* p, int value, size_t bytes) {
-    if (fails(4)) return cudaErrorUnknown;
+    if (fails(4)) return g_last = cudaErrorInvalidValue;
     std::memset(p, value, bytes);
     return cudaSuccess;
 }
@@ -116,7 +117,11 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* status)
     *status = cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = g_last;
+    g_last = cudaSuccess;
+    return e;
+}
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* blocks, const void*, int, size_t) {
     *blocks = 1;
