@@ -28,8 +28,10 @@ int set_error(int code, const std::string& msg) {
 #define VPT_CUDA(call)                                                                         \
     do {                                                                                       \
         cudaError_t e_ = (call);                                                               \
-        if (e_ != cudaSuccess)                                                                 \
+        if (e_ != cudaSuccess) {                                                               \
+            cudaGetLastError(); /* reported here, not by the next launch as well */            \
             return set_error(VPT_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        }                                                                                      \
     } while (0)
 
 template <typename T>

@@ -161,3 +161,20 @@ r.close()
 print("ok", fake.fake_bytes())
 """, tmp_path)
     assert out.split() == ["ok", "0"]
+
+
+def test_failed_copy_is_reported_once(tmp_path):
+    out = _fake_cuda.run("""
+r = Renderer(8, 8)
+r.set_frame(frame_params(C1))
+set_volume = lambda: r.set_volume_dense(np.ones((32, 32, 32), np.float32), 1 / 32, [-0.5] * 3)
+fake.fake_fail(COPY, 2)
+assert failed(set_volume)
+fake.fake_fail(COPY, 0)
+Renderer(8, 8).close()
+set_volume()
+r.launch_plain(1)
+r.close()
+print("ok")
+""", tmp_path)
+    assert out.split() == ["ok"]
