@@ -53,6 +53,13 @@ void dev_free(T** p) {
     *p = nullptr;
 }
 
+// Device memory of one call, given back on every return.
+template <typename T>
+struct Scratch {
+    T* p = nullptr;
+    ~Scratch() { dev_free(&p); }
+};
+
 // Memory for one of a volume's arrays.
 template <typename T>
 int volume_alloc(vpt::VptContextImpl* c, T** p, size_t count) {
@@ -239,9 +246,8 @@ static int finish_stencils(VptContextImpl* c, unsigned int slots) {
         c->st_values_cap = 0;
         dev_free(&c->d_st_values);
         size_t free_bytes = 0, total_bytes = 0;
-        VPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) cudaGetLastError();  // free_bytes = 0: no copy
         if (values * sizeof(float) > free_bytes / 2 || dev_alloc(&c->d_st_values, values)) {
-            cudaGetLastError();
             c->release_stencils();
             return VPT_OK;
         }
@@ -261,16 +267,16 @@ static int build_grid(VptContext* c, const float* d_dense, int nx, int ny, int n
     c->ly = (ny + 7) / 8;
     c->lz = (nz + 7) / 8;
     int64_t cells = static_cast<int64_t>(c->lx) * c->ly * c->lz;
-    int32_t* d_active = nullptr;
+    Scratch<int32_t> active;
     int rc;
-    if ((rc = volume_alloc(c, &d_active, cells)) || (rc = volume_alloc(c, &c->d_cell_maj, cells)) ||
+    if ((rc = volume_alloc(c, &active.p, cells)) || (rc = volume_alloc(c, &c->d_cell_maj, cells)) ||
         (rc = volume_alloc(c, &c->d_leaf_table, cells)))
         return rc;
-    vpt::leaf_stats(d_dense, nx, ny, nz, c->lx, c->ly, c->lz, d_active, c->d_cell_maj, 0);
+    vpt::leaf_stats(d_dense, nx, ny, nz, c->lx, c->ly, c->lz, active.p, c->d_cell_maj, 0);
     vpt::global_max(d_dense, nx, ny, nz, c->d_scratch_u32, 0);
     std::vector<int32_t> table(cells);
-    VPT_CUDA(cudaMemcpy(table.data(), d_active, cells * sizeof(int32_t), cudaMemcpyDeviceToHost));
-    dev_free(&d_active);
+    VPT_CUDA(cudaMemcpy(table.data(), active.p, cells * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    dev_free(&active.p);
     int64_t slots = 0;
     for (int64_t i = 0; i < cells; ++i) table[i] = table[i] ? static_cast<int32_t>(slots++) : -1;
     c->active_leaves = slots;
@@ -805,16 +811,16 @@ static int upload_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
     const int64_t cells = static_cast<int64_t>(lx) * ly * lz;
     dev_free(&c->d_dense);
     begin_volume(c);
-    int32_t* d_origins = nullptr;
+    Scratch<int32_t> d_origins;
     int rc;
     if ((rc = volume_alloc(c, &c->d_cell_maj, cells)) || (rc = volume_alloc(c, &c->d_leaf_table, cells)) ||
         (rc = volume_alloc(c, &c->d_leaf_values, std::max<int64_t>(slots, 1) * 512)) ||
-        (rc = volume_alloc(c, &d_origins, std::max<int64_t>(slots, 1) * 3)))
+        (rc = volume_alloc(c, &d_origins.p, std::max<int64_t>(slots, 1) * 3)))
         return rc;
     VPT_CUDA(cudaMemcpy(c->d_leaf_table, table.data(), cells * sizeof(int32_t), cudaMemcpyHostToDevice));
     if (slots > 0) {
         VPT_CUDA(cudaMemcpy(c->d_leaf_values, values, slots * 512 * sizeof(float), cudaMemcpyHostToDevice));
-        VPT_CUDA(cudaMemcpy(d_origins, origins.data(), slots * 3 * sizeof(int32_t), cudaMemcpyHostToDevice));
+        VPT_CUDA(cudaMemcpy(d_origins.p, origins.data(), slots * 3 * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
     c->lx = lx;
     c->ly = ly;
@@ -828,13 +834,16 @@ static int upload_grid(VptContextImpl* c, const std::vector<int32_t>& table, int
         box_lo[a] = info.index_min[a] - lo[a];
         box_hi[a] = info.index_max[a] - lo[a];
     }
-    vpt::leaf_box_max(c->d_leaf_values, d_origins, slots, box_lo, box_hi, c->d_scratch_u32, 0);
+    vpt::leaf_box_max(c->d_leaf_values, d_origins.p, slots, box_lo, box_hi, c->d_scratch_u32, 0);
     cudaError_t e = cudaGetLastError();
     const bool stencils = e == cudaSuccess && begin_stencils(c);
     unsigned int bits[2] = {0, 0};  // global majorant, slots of the stencil copy
     if (e == cudaSuccess) e = cudaMemcpy(bits, c->d_scratch_u32, sizeof(bits), cudaMemcpyDeviceToHost);
-    dev_free(&d_origins);
-    if (e != cudaSuccess) return set_error(VPT_ERR_CUDA, std::string("vpt_set_volume_nanovdb: ") + cudaGetErrorString(e));
+    dev_free(&d_origins.p);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return set_error(VPT_ERR_CUDA, std::string("vpt_set_volume_nanovdb: ") + cudaGetErrorString(e));
+    }
     std::memcpy(&c->global_majorant, bits, sizeof(float));
     c->active_leaves = slots;
     c->total_leaves = cells;

@@ -1,7 +1,7 @@
 """Replacing a context's volume, on a stand-in for the CUDA runtime (no GPU)."""
 import pytest
 
-from . import _fake_cuda
+from . import _fake_cuda, _nvdb
 
 SETTERS = {
     "dense": "lambda r, n: r.set_volume_dense(np.ones((n, n, n), np.float32), 1 / n, [-0.5] * 3)",
@@ -162,7 +162,6 @@ print("ok", fake.fake_bytes())
 """, tmp_path)
     assert out.split() == ["ok", "0"]
 
-
 def test_failed_copy_is_reported_once(tmp_path):
     out = _fake_cuda.run("""
 r = Renderer(8, 8)
@@ -175,6 +174,33 @@ Renderer(8, 8).close()
 set_volume()
 r.launch_plain(1)
 r.close()
+print("ok")
+""", tmp_path)
+    assert out.split() == ["ok"]
+
+
+@pytest.mark.parametrize("kind", list(SETTERS) + ["nanovdb"])
+def test_failed_calls_leak_nothing(tmp_path, kind):
+    """Whichever copy or allocation of a volume's set-up fails, destroying the context gives everything
+    back; a query of the free memory that fails costs the stencil copy alone."""
+    name = sorted(_nvdb.reference())[0]
+    path = _nvdb.fixture_path(name, tmp_path)
+    setter = SETTERS.get(kind, f"lambda r, n: r.load_nvdb({str(path)!r})")
+    out = _fake_cuda.run(f"set_volume = {setter}\n" + """
+for what in (MALLOC, COPY, MEMINFO):
+    failures = 0
+    for nth in range(1, 16):
+        r = Renderer(8, 8)
+        r.set_frame(frame_params(C1))
+        fake.fake_fail(what, nth)
+        why = failed(lambda: set_volume(r, 40))
+        fake.fake_fail(what, 0)
+        refused = failed(lambda: r.launch_plain(1))
+        assert bool(why) == bool(refused), (what, nth, why, refused)
+        failures += why is not None
+        r.close()
+        assert fake.fake_bytes() == 0, (what, nth)
+    assert (failures == 0) == (what == MEMINFO)
 print("ok")
 """, tmp_path)
     assert out.split() == ["ok"]
