@@ -216,8 +216,8 @@ static bool stencils_allowed(const VptContextImpl* c, int64_t entries) {
 // The first half, once the leaves and their table are in place: the cells' slots (and behind them, in
 // the same array, the slots' cells), their count in d_scratch_u32[1]. False where there is no room.
 static bool begin_stencils(VptContextImpl* c) {
-    const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
-    if (!stencils_allowed(c, 2 * cells + 4096)) {
+    const int64_t cells = vpt::stencil_cells(c->lx, c->ly, c->lz);
+    if (cells == 0 || !stencils_allowed(c, 2 * cells + 4096)) {
         c->release_stencils();
         return false;
     }
@@ -236,7 +236,7 @@ static bool begin_stencils(VptContextImpl* c) {
 
 // The second half: the stencils of `slots` cells.
 static int finish_stencils(VptContextImpl* c, unsigned int slots) {
-    const int64_t cells = static_cast<int64_t>(c->lx + 1) * (c->ly + 1) * (c->lz + 1);
+    const int64_t cells = vpt::stencil_cells(c->lx, c->ly, c->lz);
     const int64_t values = static_cast<int64_t>(std::max(slots, 1u)) * 4096;
     if (!stencils_allowed(c, 2 * cells + values)) {
         c->release_stencils();

@@ -124,6 +124,12 @@ struct VptContextImpl {
 };
 
 int ctx_set_error(int code, const char* msg);
+// Cells of the stencil copy of a grid of lx x ly x lz leaf cells, or 0 where their indices, kept in 32
+// bits by the lookups and by the list of slots, would not fit (thin grids of up to 2^30 leaf cells).
+inline int64_t stencil_cells(int32_t lx, int32_t ly, int32_t lz) {
+    const int64_t cells = (static_cast<int64_t>(lx) + 1) * (static_cast<int64_t>(ly) + 1) * (static_cast<int64_t>(lz) + 1);
+    return cells <= INT32_MAX ? cells : 0;
+}
 int fill_trace_params(VptContextImpl* c, TraceParams* tp);
 int persistent_grid(VptContextImpl* c, int threads, const void* kernel, size_t smem);
 // LCG jump (multiplier, increment) that advances a PCG32 state by `delta` draws.
