@@ -12,7 +12,7 @@ tracer to reach relMSE 1e-3 against a 16384-spp FP64 image on the 256x256 dense 
 `--config c4` times the 16-scene batch (one CUDA graph per step), `--config c5` the 2048^2 /
 1024^3 stress scene; `--nrc-frames N` runs only the radiance-cache frame loop and `--mlp` only
 the cache's MLP kernels (profiling); `--tracker wavefront` times the wavefront form of the plain
-tracker instead of the persistent megakernel.
+tracker instead of the persistent one (work queues).
 
 `--impl reference` times the reference's per-path CPU algorithm on the host cores. The reference's
 own implementation (OptiX raygen + tiny-cuda-nn) cannot be built on this platform, so the arm runs
@@ -552,7 +552,7 @@ def main():
     ap.add_argument("--no-nrc", action="store_true", help="skip the NRC-vs-plain equal-error comparison")
     ap.add_argument("--no-mlp", action="store_true", help="skip the MLP kernel figures of the default line")
     ap.add_argument("--tracker", default="megakernel", choices=["megakernel", "wavefront"],
-                    help="plain tracker: the persistent megakernel (default) or the wavefront form")
+                    help="plain tracker: the persistent one with work queues ('megakernel', default) or the wavefront form")
     ap.add_argument("--mlp", action="store_true",
                     help="profiling run: only the cache's MLP kernels (inference and training steps)")
     ap.add_argument("--nrc-frames", type=int, default=0,

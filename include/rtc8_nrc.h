@@ -65,6 +65,11 @@ typedef struct NrcHandle NrcHandle;
 
 /* Fills `cfg` with the reference's settings for the given encoding. */
 void nrc_default_config(int32_t encoding, NrcConfig* cfg);
+/* A cache holds four FP32 copies of its parameters and two of their gradients. With the hash grid it also
+ * holds 16 MB for the features of a training step's records (without room for them the training kernel
+ * gathers the features itself), and the caches of a device share a pool of 76 MB workspaces for large inference
+ * batches, one reserved with the first cache and one more for each stream that infers at the same time; the
+ * pool is given back with the last of them. */
 int nrc_create(const NrcConfig* cfg, NrcHandle** out);
 int nrc_destroy(NrcHandle* h);
 const char* nrc_last_error(void);

@@ -408,7 +408,7 @@ int vpt_set_leaf_staging(VptContext* ctx, int32_t min_lanes);
 /* Launch shape of the persistent trackers: CTAs per SM, threads per CTA (a multiple of 32 up to
  * 128), and, with leaf staging only, the number of parked lanes of a warp that triggers its joint
  * event phase (the default tracker has work queues instead); 0 = defaults: three CTAs of 256 threads
- * per SM, with leaf staging as many of 128 as fit and 16 parked lanes. Contexts whose launches run
+ * per SM (two with meshes), with leaf staging as many of 128 as fit and 16 parked lanes. Contexts whose launches run
  * concurrently on one GPU (several scenes at once) do better with 128-thread CTAs, which can share
  * an SM. */
 int vpt_set_launch_shape(VptContext* ctx, int32_t ctas_per_sm, int32_t threads_per_cta,

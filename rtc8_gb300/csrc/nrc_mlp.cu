@@ -612,8 +612,10 @@ __global__ void __launch_bounds__(kEncodeThreads, 1) grid_encode_kernel(const Ne
 // one group runs its epilogue or encodes its next input, the tensor cores serve another: G tiles
 // in flight per SM instead of one per CTA. A group reuses its input tile's shared memory for the
 // hidden activations (a layer's MMA has completed before its epilogue overwrites the operand).
-// What bounds it (one tile of the volume network, 10.4k cycles with four groups on an SM): the tensor
-// pipe at N = 64 (29 MMAs at 78-90 cycles each), then the encoder (1.9k). Encoder warps of their own
+// Where its time goes (one tile of the volume network, 10.4k cycles with four groups on an SM, 2.7k per
+// tile of the SM): the products (29 MMAs, 78-90 cycles each; back to back, with both operands in shared
+// memory, an MMA of this width takes 48; with A in tensor memory, as 20 of them have it, that
+// rate is not measured), then the encoder (1.9k). Encoder warps of their own
 // were slower (4 M volume queries 304 -> 354 us). Small batches are bound by latency: one bulk copy
 // brings the weights while the first queries load, and the tiles go to the SMs in turn (us, before
 // this / now: up to 24,000 queries volume 10.3 / 8.2, reference 8.2 / 6.2, hash grid 22.6 / 12.4;

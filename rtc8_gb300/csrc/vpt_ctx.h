@@ -97,7 +97,7 @@ struct VptContextImpl {
 
     // neural-radiance-cache render/training buffers (allocated on first use)
     // wavefront tracer of the plain path (allocated on first use)
-    int32_t tracker = 0;                // 0 = persistent megakernel, 1 = wavefront
+    int32_t tracker = 0;                // 0 = persistent (work queues), 1 = wavefront
     int32_t wf_slots_per_sm = 0, wf_pass_steps = 0, wf_track_ctas_per_sm = 0;
     WfBuffers wf;
     uint32_t* wf_pinned = nullptr;

@@ -287,9 +287,11 @@ __device__ __forceinline__ float sample_trilinear(const Grid& g, V3 xyz, LeafCac
 // instructions around them: the leaf layout reads four sectors with eight loads (two table reads
 // and 32 bounds checks more for the third of the lookups that straddle leaves, a second code path
 // that nearly every warp iteration also executes). Sparse 512^3 at 256^2 x 16 spp: warp
-// instructions 3.33 -> 2.33 G, L1 sectors 209 -> 59 M; launches: 1024^2 x 16 spp 33.0 -> 26.5 ms,
-// the 1024^3 scene 22.4 -> 17.5 ms, dense 64^3 at 256^2 x 16 spp 1.14 -> 0.94 ms, reference rules
-// 6.68 -> 5.00 ms, a radiance-cache frame 5.05 -> 4.35 ms.
+// instructions 3.33 -> 2.33 G, L1 sectors 209 -> 59 M (in a tracker with one path per lane, as it was
+// then). In the tracker with work queues, ms per launch through the leaves / through the copy: sparse
+// 512^3 at 1024^2 x 16 spp 27.4 / 17.7, the 1024^3 scene at 2048^2 x 4 spp 15.6 / 10.9, dense 64^3 at
+// 256^2 x 16 spp 0.97 / 0.80 and x 1 spp 0.57 / 0.50, reference rules 4.53 / 3.34, a radiance-cache
+// frame 3.35 / 2.76; with meshes, 512^2 x 4 spp: the room 7.57 / 6.59, with two spheres 12.2 / 10.0.
 __device__ __forceinline__ float sample_stencil(const Grid& g, V3 xyz, LeafCache& cache) {
     Stencil s;
     const float fi = floorf(xyz.x), fj = floorf(xyz.y), fk = floorf(xyz.z);

@@ -15,10 +15,11 @@
 //
 // What bounded the form that keeps a path in each lane was divergence: its warps ran every event
 // for the few lanes that happened to have it (5.4 threads per warp instruction on the sparse
-// 512^3 scene; here 27 of 32 lanes in a tracking step and 25 to 28 in an event batch while there is
-// work). CTA barriers between a tracking and an event phase (17 barrier stalls per issue), one
+// 512^3 scene, here 13.8; 27 of 32 lanes hold work in a tracking step and 25 to 28 in an event batch
+// while there is any, and diverge inside it). CTA barriers between a tracking and an event phase (17 barrier stalls per issue), one
 // queue per CTA of 128 or of 768 threads, and 4 CTAs per SM at 64 registers were all slower. ms per
-// launch, lane-per-path form against this one: 1024^2 x 16 spp sparse 512^3 23.6 -> 16.0, 2048^2 x
+// launch, lane-per-path form against this one, both with the stencil copy and one seed's clouds (another
+// seed's or another GPU's sparse launch takes 15.5 to 20.7): 1024^2 x 16 spp sparse 512^3 23.6 -> 16.0, 2048^2 x
 // 4 spp 1024^3 17.4 -> 11.9, dense 64^3 at 256^2 x 16 spp 0.89 -> 0.74 and x 1 spp 0.53 -> 0.45,
 // reference rules 256^2 x 8 spp 4.2 -> 2.9, a radiance-cache frame 4.27 -> 2.99. With meshes, 512^2 x
 // 4 spp: the room 23.9 -> 6.7, with two spheres through the BVH 30.5 -> 10.2 (bound by instruction

@@ -18,8 +18,8 @@
 //     longest segment of the image.
 // Queues are compacted with warp-aggregated atomics; the host issues passes until the tracking
 // queue stays empty after an event pass. Per path the random numbers are drawn in exactly the
-// order of the persistent megakernel (vpt_tracer.cu), so both produce the same decisions.
-// This unit is compiled without multiply-add contraction, like the megakernel.
+// order of the tracker with work queues (vpt_queues.cu), so both produce the same decisions.
+// This unit is compiled without multiply-add contraction, like that one.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -67,7 +67,7 @@ __device__ __forceinline__ uint32_t make_flags(uint32_t st, uint32_t end, uint32
     return st | (end << 8) | bits;
 }
 
-// Majorant-grid DDA (the megakernel's definition, vpt_tracer.cu).
+// Majorant-grid DDA (the definition of vpt_track.cuh).
 struct Dda {
     int cell[3];
     int step[3];

@@ -230,7 +230,7 @@ class Renderer:
         check(self.lib.vpt_set_frame_params(self.ctx, C.byref(p)), "vpt_set_frame_params")
 
     def set_tracker(self, kind: int = 0, slots_per_sm: int = 0, pass_steps: int = 0, track_ctas_per_sm: int = 0) -> None:
-        """0 = persistent megakernel (default), 1 = wavefront; see vpt_set_tracker."""
+        """0 = persistent tracker with work queues (default), 1 = wavefront; see vpt_set_tracker."""
         check(self.lib.vpt_set_tracker(self.ctx, kind, slots_per_sm, pass_steps, track_ctas_per_sm), "vpt_set_tracker")
 
     def set_leaf_staging(self, min_lanes: int) -> None:
